@@ -69,15 +69,16 @@ def sumfac_inputs(geo: Geometry, K_max: int, gamma: float, radial_pad: int = 40,
     N_t1, N_u1, N_y2 = s["N_t1"], s["N_u1"], s["N_y2"]
     L_triplets = np.zeros((N_L, 3))
     qi_valid = -np.ones((NQ, N_L))
-    P_loss_p1 = np.zeros((N_t1, N_u1, N_L))
-    P_loss_p2 = np.zeros((N_y2, N_L))
+    # column-major, as MATLAB holds them: compute_R passes them on without a copy
+    P_loss_p1 = np.zeros((N_t1, N_u1, N_L), order="F")
+    P_loss_p2 = np.zeros((N_y2, N_L), order="F")
     if packed:
         P_gain_p1 = P_gain_p2 = None
         cols1: list[np.ndarray] = []  # per channel [n_qi, N_t1, N_u1]
         cols2: list[np.ndarray] = []  # per channel [n_qi, N_y2]
     else:
-        P_gain_p1 = np.zeros((N_t1, N_u1, NQ, N_L))
-        P_gain_p2 = np.zeros((N_y2, NQ, N_L))
+        P_gain_p1 = np.zeros((N_t1, N_u1, NQ, N_L), order="F")
+        P_gain_p2 = np.zeros((N_y2, NQ, N_L), order="F")
 
     # SH values at phi = 0 on the two patches' polar grids (:143-145, :156-158)
     y1 = qu1.x[None, :] * qt1.x[:, None]  # [N_t1, N_u1]

@@ -43,6 +43,11 @@ struct DevOp {
     int n_l;
 };
 
+// The fast FP64 pair routine sums a row's slices in up to kRowParts consecutive parts, each on its own,
+// and add the parts in order.  A small batch gives the parts to different warps; the sum is the same bit for bit.
+constexpr int kRowParts = 8;
+__host__ __device__ constexpr int row_part(int n, int g) { return n * g / kRowParts; }  // part g: [row_part(n, g), row_part(n, g + 1))
+
 // Batches of at most this many cells take the few-cell kernel (few_kernels.cuh).
 constexpr int kFewCells = 8;
 

@@ -1,5 +1,6 @@
 // inst.cuh -- the body of one per-K translation unit (included by inst_k<K>.cu with CF_K defined).
 #pragma once
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -185,34 +186,50 @@ static inline UnitPlan plan_units(int64_t n_cells, int64_t ctas) {
     return {(int)n_ht, (int)n_whole, split, (int)(n_whole + rem * split)};
 }
 
-template <int K, int W, bool EXACT, bool JV, bool RG, typename T = double, bool SPLIT = false>
+template <int K, int W, bool EXACT, bool JV, bool RG, typename T = double, bool SPLIT = false, bool CM = false>
 static LaunchResult launch_pair(const LaunchArgs& a) {
     const int M = a.op.n_q * K;
-    const size_t smem = pair_smem_bytes<K, T>(M, W, JV, RG);
+    size_t smem = pair_smem_bytes<K, T>(M, W, JV, RG,
+                                       sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(K, JV));
+    int share = 0;
+    if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT) {
+        // a batch of fewer half-tiles than SMs: room behind the tile for the part sums of units with fewer
+        // items than warps (a larger one keeps its shared memory for a second CTA on the SM)
+        constexpr size_t per_item = sizeof(double) * kRowParts * K * 32;
+        if ((a.n_cells + kTileCells - 1) / kTileCells < a.n_sms && smem + 256 <= a.max_smem) {
+            share = (int)std::min<size_t>(W - 1, (a.max_smem - 256 - smem) / per_item);
+            smem += share * per_item;
+        }
+    }
     if (smem + 256 > a.max_smem || a.counter == nullptr || a.pitems == nullptr) return {-1, 0, cudaSuccess, PATH_PAIR};
     static_assert(!SPLIT || (!EXACT && !JV && !RG && K % 2 == 0), "the split variant is the fast Q form");
-    auto kern = af_pair_kernel<K, W, EXACT, JV, RG, T, SPLIT>;
+    auto kern = af_pair_kernel<K, W, EXACT, JV, RG, T, SPLIT, CM>;
     int per_sm = 0;
     cudaError_t e = resident_ctas((const void*)kern, W * 32, smem, &per_sm);
     if (e != cudaSuccess) return {5, 0, e, PATH_PAIR};
     if (per_sm < 1) return {-1, 0, cudaSuccess, PATH_PAIR};
     const int64_t ctas = (int64_t)per_sm * a.n_sms;
     if ((a.n_cells + kTileCells - 1) / kTileCells * 16 > INT32_MAX) return {2, 0, cudaSuccess, PATH_PAIR};
-    const UnitPlan up = plan_units(a.n_cells, ctas);
-    PairSched sc{a.pbin_begin, a.pbin_item, a.pitems, up.n_ht, up.n_whole, up.split, up.n_units, a.counter};
+    // sixteenths where their few items are shared out by parts (L = 12, K = 5, 2048 cells: 958 against 1038 us;
+    // unshared ones are slower: L = 8, K = 6, 4096 cells 887 against 811 us)
+    const UnitCuts cuts = cut_units((a.n_cells + kTileCells - 1) / kTileCells, ctas, share > 0);
+    PairSched sc{a.pbin_begin, a.pbin_item, a.pitems, cuts, a.counter, share};
     e = cudaMemsetAsync(a.counter, 0, sizeof(int), a.stream);
     if (e != cudaSuccess) return {5, 0, e, PATH_PAIR};
-    const unsigned grid = (unsigned)(up.n_units < ctas ? up.n_units : ctas);
+    const unsigned grid = (unsigned)std::min<int64_t>(cuts.n_units, ctas);
     const T* fT;
     const T* vT;
-    if constexpr (sizeof(T) == 8) {
+    if constexpr (CM) {
+        fT = a.f_cm;
+        vT = a.v_cm;
+    } else if constexpr (sizeof(T) == 8) {
         fT = a.fT;
         vT = a.vT;
     } else {
         fT = a.fT32;
         vT = a.vT32;
     }
-    kern<<<grid, W * 32, smem, a.stream>>>(a.op, sc, fT, vT, a.QT);
+    kern<<<grid, W * 32, smem, a.stream>>>(a.op, sc, fT, vT, CM ? a.q_cm : a.QT, (long long)a.n_cells);
     e = cudaGetLastError();
     return {e == cudaSuccess ? 0 : 5, 1, e, SPLIT ? PATH_PAIR_SPLIT : (RG ? PATH_PAIR_L1 : PATH_PAIR)};
 }
@@ -426,6 +443,17 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
             return a.what == OP_AF || a.what == OP_JV ? launch_few_exact<K>(a) : LaunchResult{-1, 0, cudaSuccess, PATH_FEW};
         return a.what == OP_RF ? launch_few<K, true>(a) : launch_few<K, false>(a);
     }
+    if (a.pair_cm) {
+        if constexpr (K <= 8) {
+            if (a.what != OP_RF && !a.exact && !a.f32) {
+                const LaunchResult r =
+                    a.what == OP_JV ? launch_pair<K, pair_W(K, true), false, true, false, double, false, true>(a)
+                                    : launch_pair<K, pair_W(K), false, false, false, double, false, true>(a);
+                if (r.status != -1) return r;
+            }
+        }
+        return {8, 0, cudaSuccess, PATH_PAIR};
+    }
     if (a.ss) {
         if (a.what != OP_AF || a.exact || a.f32) return {8, 0, cudaSuccess, PATH_TILE};
         if constexpr (K % 2 == 0 && K <= 8) {
@@ -503,15 +531,17 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
             LaunchResult r;
             if (a.path == PATH_PAIR_L1) {
                 if (jv)
-                    r = a.exact ? launch_pair<K, 8, true, true, true>(a) : launch_pair<K, 8, false, true, true>(a);
+                    r = a.exact ? launch_pair<K, pair_W(K, true), true, true, true>(a) : launch_pair<K, pair_W(K, true), false, true, true>(a);
                 else
-                    r = a.exact ? launch_pair<K, 8, true, false, true>(a) : launch_pair<K, 8, false, false, true>(a);
+                    r = a.exact ? launch_pair<K, pair_W(K), true, false, true>(a) : launch_pair<K, pair_W(K), false, false, true>(a);
             } else {
                 if (jv)
-                    r = a.exact ? launch_pair<K, 8, true, true, false>(a) : launch_pair<K, 8, false, true, false>(a);
+                    r = a.exact ? launch_pair<K, pair_W(K, true), true, true, false>(a) : launch_pair<K, pair_W(K, true), false, true, false>(a);
                 else
-                    r = a.exact ? launch_pair<K, 8, true, false, false>(a) : launch_pair<K, 8, false, false, false>(a);
+                    r = a.exact ? launch_pair<K, pair_W(K), true, false, false>(a) : launch_pair<K, pair_W(K), false, false, false>(a);
             }
+            if (r.status == -1 && a.path != PATH_PAIR_L1 && jv && !a.exact && pair_W(K, true) > 8)
+                r = launch_pair<K, 8, false, true, false>(a);  // fewer copies of R_t
             if (r.status != -1) return r;
             if (a.path != PATH_AUTO) return {8, 0, cudaSuccess, a.path};
         }

@@ -65,6 +65,8 @@ struct LaunchArgs {
     // with few: the exact form of any number of cells on the row kernel (one CTA per (q1, pair of cells), on the
     // cell-major arrays), the exact route where the batch kernels' register tiles do not fit (K > 8)
     bool rows = false;
+    // the fast FP64 forms on the pair kernel, on the cell-major arrays f_cm, v_cm, q_cm
+    bool pair_cm = false;
 };
 
 // Status codes mirror cf_status: 0 ok, 5 CUDA error, 8 unsupported, 2 shape.
@@ -84,6 +86,17 @@ CF_DECLARE_K(13) CF_DECLARE_K(14) CF_DECLARE_K(15) CF_DECLARE_K(16)
 // Lanes per cell (P) of the fast kernels: the K x K Phi accumulator is split over P lanes by
 // k3 column once it no longer fits one lane's registers.
 constexpr int af_P(int K) { return K <= 8 ? 1 : (K <= 12 ? 2 : 4); }
+// Warps per CTA of the FP64 pair kernel: as many as the registers of a whole Phi per lane leave (Q at K = 5: 128 a
+// lane; K = 6, and J.v at K = 5: 168; else 255, or several CTAs on an SM below K = 5).
+constexpr int pair_W(int K, bool jv = false) { return K == 5 ? (jv ? 12 : 16) : (K == 6 && !jv ? 12 : 8); }
+// Shared memory of a warp: R_t and, where registers are short (the 16- and 12-warp Q forms), the row sums.
+constexpr bool pair_sums_shared(int K, bool jv) { return pair_W(K, jv) > 8 && !jv; }
+constexpr int pair_warp_doubles(int K, bool jv) { return (K * K * K + 1) / 2 * 2 + (pair_sums_shared(K, jv) ? K * 32 : 0); }
+// Whether the FP64 pair kernel's 16-cell tile of f (and v) fits beside its warps' copies of R_t.
+constexpr bool pair_fits(int n_q, int K, bool jv, size_t max_smem) {
+    return K <= 8 && sizeof(double) * ((size_t)(jv ? 2 : 1) * n_q * K * 16 + (size_t)pair_W(K, jv) * pair_warp_doubles(K, jv)) +
+                             256 <= max_smem;
+}
 constexpr int jv_P(int K) { return K <= 6 ? 1 : (K <= 8 ? 2 : 4); }
 
 }  // namespace cf

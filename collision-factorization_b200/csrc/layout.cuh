@@ -57,6 +57,29 @@ static __global__ void __launch_bounds__(256) unpack_tiles_kernel(const double* 
     }
 }
 
+// R in FP32; at K = 8 (RT not null) also R_t as [k1][8 k2 + k3], and that split into BF16 hi + lo (each rounded to
+// nearest even), [t][hi, lo][k1][8 k2 + k3].
+__device__ __forceinline__ unsigned short bf16_round(float x) {
+    uint32_t u = __float_as_uint(x);
+    u += 0x7fffu + ((u >> 16) & 1u);
+    return (unsigned short)(u >> 16);
+}
+static __global__ void __launch_bounds__(256) derive_r_kernel(const double* __restrict__ R, float* __restrict__ R32,
+                                                              double* __restrict__ RT, unsigned short* __restrict__ RTbf,
+                                                              size_t n) {
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const double r = R[i];
+    R32[i] = (float)r;
+    if (RT == nullptr) return;
+    const size_t t = i / 512;
+    const int e = (int)(i % 512), j = (e % 8) * 64 + (e / 8) % 8 * 8 + e / 64;
+    RT[t * 512 + j] = r;
+    const unsigned short hi = bf16_round((float)r);
+    RTbf[t * 1024 + j] = hi;
+    RTbf[t * 1024 + 512 + j] = bf16_round((float)(r - (double)__uint_as_float((uint32_t)hi << 16)));
+}
+
 // FP64 FMA throughput probe: kProbeChains independent DFMA chains per thread.
 constexpr int kProbeChains = 8;
 static __global__ void __launch_bounds__(256) fp64_fma_probe_kernel(double* sink, int iters, double a) {

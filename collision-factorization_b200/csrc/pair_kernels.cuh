@@ -11,6 +11,13 @@
 // warp-uniform shared loads, and each f row read by a half-warp is one 128-byte wavefront.  Rows
 // without a mirror (m1 = 0, or a structure mismatch) run with the upper half idle.
 //
+// What bounds it: shared-memory wavefronts (83 % of peak at K = 5; FP64 pipe 49 %) -- 2 K loads an entry and one
+// wavefront per R_t element -- and, before a row's slices were read ahead and the CTA had more warps than 8,
+// the L2 round trips between slices.  B200, folded, L = 12, K = 5, 2048 cells: 8 warps 1360 us, 16 warps and
+// read-ahead 1045 us, with the last half-tiles in sixteenths 958 us.  Small batches are bound by one row's
+// slices in sequence and by launches: L = 4, K = 5, 100 cells, plain: layout passes and whole rows 35.7 us,
+// cell-major with rows in parts 18.0 us.
+//
 // The rest follows tile_kernels.cuh: 16-cell half-tile resident in shared memory, R_t staged per
 // warp with cp.async, persistent CTAs pulling whole half-tiles and then binned half-tiles from a
 // device counter, warps pulling pair items from a shared counter.
@@ -18,6 +25,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "tile_kernels.cuh"
 
 namespace cf {
@@ -26,8 +34,9 @@ struct PairSched {
     const int* bin_begin;  // bins over pair items: 0 = all (heaviest first), 1..4, 5..20
     const int* bin_item;   // item indices
     const int2* items;     // (qa, qb); qb = -1 for a row without a mirror
-    int n_ht, n_whole, split, n_units;
+    UnitCuts cuts;
     int* counter;
+    int share;  // items per unit that the shared part sums have room for (0: none)
 };
 
 template <int K, typename T = double>
@@ -49,9 +58,14 @@ __device__ __forceinline__ const float* r_tensor<float>(const DevOp& op) { retur
 // of the slice), which keeps the K^3 step off the shared-memory wavefront budget.
 // T = double: the FP64 forms (accumulating from the caller's Q).  T = float: the FP32 form (f, R,
 // Phi and the per-row sums in FP32; the FP32 result is added to the caller's FP64 Q at the end).
-template <int K, bool EXACT, bool JV, bool RG, typename T = double>
+// CM: qtc points at the lane's cell in the caller's cell-major Q, read and written where `live`; else at its
+// column of the tiled Q.  `part`: -1 contracts the whole row pair into Q; a number returns that part's sum in
+// `sum` (fast FP64 forms) and leaves Q alone.
+// TS: the row sums between parts are kept in the warp's shared memory, behind its R_t.
+template <int K, bool EXACT, bool JV, bool RG, typename T = double, bool CM = false, bool TS = false>
 __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* __restrict__ fs,
-                                          const T* __restrict__ vs, T* rb, double* qtc, int lane) {
+                                          const T* __restrict__ vs, T* rb, double* qtc, int lane, bool live = true,
+                                          int part = -1, double* sum = nullptr) {
     static_assert(!EXACT || sizeof(T) == 8, "the exact order is FP64");
     constexpr bool F64 = sizeof(T) == 8;
     const int half = lane >> 4;
@@ -59,19 +73,78 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
     const bool active = half == 0 || item.y >= 0;
     const int q1 = half == 0 ? item.x : (item.y >= 0 ? item.y : item.x);
 
+    constexpr bool PARTS = F64 && !EXACT;
     T acc[K];
+    double tot[PARTS && !TS ? K : 1];
+    double* ts = TS ? reinterpret_cast<double*>(rb) + RPair<K, T>::SIZE + lane : nullptr;
+    if constexpr (PARTS) {
 #pragma unroll
-    for (int k1 = 0; k1 < K; ++k1) acc[k1] = (F64 && active) ? (T)qtc[(size_t)(q1 * K + k1) * CF_TILE] : (T)0;
+        for (int k1 = 0; k1 < K; ++k1) {
+            const double q = part < 0 && active && live ? qtc[q_off<K, CM>(q1, k1, op.n_q)] : 0.0;
+            if constexpr (TS)
+                ts[k1 * 32] = q;
+            else
+                tot[k1] = q;
+            acc[k1] = (T)0;
+        }
+    } else {
+#pragma unroll
+        for (int k1 = 0; k1 < K; ++k1)
+            acc[k1] = (F64 && active && live) ? (T)qtc[q_off<K, CM>(q1, k1, op.n_q)] : (T)0;
+    }
 
     // slices of qa and qb correspond one to one (same t, same length)
     const int sa0 = op.q1_begin[item.x], sa1 = op.q1_begin[item.x + 1];
     const int sb0 = item.y >= 0 ? op.q1_begin[item.y] : sa0;
-    for (int i = 0; i < sa1 - sa0; ++i) {
-        const int sa = sa0 + i, sb = sb0 + i;
-        const int t = op.slice_t[sa];
-        const int ea = op.slice_e[sa], n_e = op.slice_e[sa + 1] - ea;
-        const int eb_ = op.slice_e[sb];
-        const int my_e0 = half == 0 ? ea : eb_;
+    // a slice's triplet, entry range and first 16 entries are read while the slice before it is
+    // contracted (each is an L2 round trip, longer than a short slice's arithmetic)
+    const int n_s = sa1 - sa0;
+    int nx_t = 0, nx_n = 0, nx_e0 = 0;
+    uint32_t nx_q23 = 0;
+    double nx_g = 0.0;
+    auto range = [&](int i) {
+        nx_t = __ldg(op.slice_t + sa0 + i);
+        const int ea = __ldg(op.slice_e + sa0 + i), eb_ = __ldg(op.slice_e + sb0 + i);
+        nx_n = __ldg(op.slice_e + sa0 + i + 1) - ea;
+        nx_e0 = half == 0 ? ea : eb_;
+    };
+    auto entries = [&]() {
+        nx_q23 = 0;
+        nx_g = 0.0;
+        if (c < nx_n && active) {
+            nx_q23 = __ldg(op.e_q23 + nx_e0 + c);
+            nx_g = __ldg(op.e_g + nx_e0 + c);
+        }
+    };
+    const int i_lo = PARTS && part >= 0 ? row_part(n_s, part) : 0;
+    const int i_hi = PARTS && part >= 0 ? row_part(n_s, part + 1) : n_s;
+    int g_end = i_hi, g_no = 0;  // end and number of the part in work
+    if constexpr (PARTS)
+        if (part < 0) g_end = row_part(n_s, 1);
+    if (i_lo < i_hi) {
+        range(i_lo);
+        entries();
+    }
+    for (int i = i_lo; i < i_hi; ++i) {
+        if constexpr (PARTS) {
+            if (part < 0)
+                while (i == g_end) {
+#pragma unroll
+                    for (int k1 = 0; k1 < K; ++k1) {
+                        if constexpr (TS)
+                            ts[k1 * 32] += acc[k1];
+                        else
+                            tot[k1] += acc[k1];
+                        acc[k1] = (T)0;
+                    }
+                    ++g_no;
+                    g_end = row_part(n_s, g_no + 1);
+                }
+        }
+        const int t = nx_t, n_e = nx_n, my_e0 = nx_e0;
+        const uint32_t q23_0 = nx_q23;
+        const double g_0 = nx_g;
+        if (i + 1 < i_hi) range(i + 1);
 
         const T* __restrict__ Rt = r_tensor<T>(op) + (size_t)t * K * K * K;
         if constexpr (RG) {
@@ -99,11 +172,15 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
 
         for (int e0 = 0; e0 < n_e; e0 += 16) {
             const int n = min(16, n_e - e0);
-            uint32_t my_q23 = 0;
-            double my_g = 0.0;
-            if (c < n && active) {
-                my_q23 = __ldg(op.e_q23 + my_e0 + e0 + c);
-                my_g = __ldg(op.e_g + my_e0 + e0 + c);
+            uint32_t my_q23 = q23_0;
+            double my_g = g_0;
+            if (e0 > 0) {
+                my_q23 = 0;
+                my_g = 0.0;
+                if (c < n && active) {
+                    my_q23 = __ldg(op.e_q23 + my_e0 + e0 + c);
+                    my_g = __ldg(op.e_g + my_e0 + e0 + c);
+                }
             }
             for (int j = 0; j < n; ++j) {
                 const uint32_t q23 = __shfl_sync(0xffffffffu, my_q23, j + 16 * half);
@@ -156,6 +233,7 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
                 }
             }
         }
+        if (i + 1 < i_hi) entries();
         if constexpr (!RG) {
             cp_async_wait_all();
             __syncwarp();
@@ -204,6 +282,25 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
                         acc[2 * h + 1] = fma(r.y, phi[a][b], acc[2 * h + 1]);
                     }
                 }
+        } else if constexpr (F64 && !RG) {
+            // odd K: R_t's elements in order, two per load (a broadcast load costs the same wavefronts for
+            // 16 bytes as for 8)
+            double2 r = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int b = 0; b < K; ++b)
+#pragma unroll
+                for (int a = 0; a < K; ++a)
+#pragma unroll
+                    for (int k1 = 0; k1 < K; ++k1) {
+                        const int e = k1 + K * a + K * K * b;
+                        if (e % 2 == 0) {
+                            if (e + 1 < K * K * K)
+                                r = *reinterpret_cast<const double2*>(rsrc + e);
+                            else
+                                r.x = rsrc[e];
+                        }
+                        acc[k1] = fma(e % 2 == 0 ? r.x : r.y, phi[a][b], acc[k1]);
+                    }
         } else {
 #pragma unroll
             for (int b = 0; b < K; ++b)
@@ -216,10 +313,19 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
                     }
         }
     }
-    if (active) {
+    if constexpr (PARTS) {
+        if (part >= 0) {
+#pragma unroll
+            for (int k1 = 0; k1 < K; ++k1) sum[k1] = acc[k1];
+            return;
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < K; ++k1)
+            if (active && live) qtc[q_off<K, CM>(q1, k1, op.n_q)] = (TS ? ts[k1 * 32] : tot[TS ? 0 : k1]) + acc[k1];
+    } else if (active && live) {
 #pragma unroll
         for (int k1 = 0; k1 < K; ++k1) {
-            double* out = qtc + (size_t)(q1 * K + k1) * CF_TILE;
+            double* out = qtc + q_off<K, CM>(q1, k1, op.n_q);
             *out = F64 ? (double)acc[k1] : *out + (double)acc[k1];
         }
     }
@@ -380,10 +486,12 @@ __device__ __forceinline__ void pair_split_item(const DevOp& op, int2 item, cons
 }
 
 // fT, vT: tiled cells in T (FP64 tiles for the FP64 forms, FP32 tiles for the FP32 form); QT: FP64.
-template <int K, int W, bool EXACT, bool JV, bool RG, typename T = double, bool SPLIT = false>
-__global__ void __launch_bounds__(W * 32, 1)
+// CM: fT, vT, QT are the caller's cell-major arrays of n_cells cells (FP64 forms).  sc.share: where a unit has
+// fewer items than warps, the warps take its (item, part) pairs and the parts are added from shared memory.
+template <int K, int W, bool EXACT, bool JV, bool RG, typename T = double, bool SPLIT = false, bool CM = false>
+__global__ void __launch_bounds__(W * 32, sizeof(T) == 8 && K <= 4 && !RG ? 2 : 1)
     af_pair_kernel(DevOp op, PairSched sc, const T* __restrict__ fT, const T* __restrict__ vT,
-                   double* __restrict__ QT) {
+                   double* __restrict__ QT, long long n_cells) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* smem = reinterpret_cast<T*>(smem_raw);
     __shared__ int s_unit, s_next;
@@ -391,7 +499,9 @@ __global__ void __launch_bounds__(W * 32, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     T* fs = smem;
     T* vs = JV ? smem + (size_t)M * kTileCells : nullptr;
-    T* rb = smem + (size_t)(JV ? 2 : 1) * M * kTileCells + (size_t)warp * RPair<K, T>::SIZE;
+    constexpr bool TS = sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(K, JV);
+    constexpr int WB = RPair<K, T>::SIZE + (TS ? K * 32 : 0);  // a warp's elements
+    T* rb = smem + (size_t)(JV ? 2 : 1) * M * kTileCells + (size_t)warp * WB;
     constexpr int PER16 = 16 / (int)sizeof(T);    // elements per 16-byte copy
     constexpr int CPR = kTileCells / PER16;       // 16-byte copies per 16-cell row
     int staged = -1;
@@ -400,28 +510,27 @@ __global__ void __launch_bounds__(W * 32, 1)
         if (tid == 0) s_unit = atomicAdd(sc.counter, 1);
         __syncthreads();
         const int u = s_unit;
-        if (u >= sc.n_units) break;
+        if (u >= sc.cuts.n_units) break;
         int ht, bin;
-        if (u < sc.n_whole) {
-            ht = u;
-            bin = 0;
-        } else {
-            const int v = u - sc.n_whole;
-            ht = sc.n_whole + v / sc.split;
-            bin = bin_base(sc.split) + v % sc.split;
-        }
+        unit_of(sc.cuts, u, ht, bin);
         const size_t tile_base = (size_t)(ht >> 1) * M * CF_TILE + (size_t)(ht & 1) * kTileCells;
+        const long long cell0 = (long long)ht * kTileCells;
         if (ht != staged) {
-            const T* srcf = fT + tile_base;
-            for (int i = tid; i < M * CPR; i += W * 32) {
-                const int r = i / CPR, w = (i % CPR) * PER16;
-                cp_async16(fs + r * kTileCells + w, srcf + (size_t)r * CF_TILE + w);
-            }
-            if constexpr (JV) {
-                const T* srcv = vT + tile_base;
+            if constexpr (CM) {
+                stage_cells<K>(fs, fT, op.n_q, cell0, n_cells, tid, W * 32);
+                if constexpr (JV) stage_cells<K>(vs, vT, op.n_q, cell0, n_cells, tid, W * 32);
+            } else {
+                const T* srcf = fT + tile_base;
                 for (int i = tid; i < M * CPR; i += W * 32) {
                     const int r = i / CPR, w = (i % CPR) * PER16;
-                    cp_async16(vs + r * kTileCells + w, srcv + (size_t)r * CF_TILE + w);
+                    cp_async16(fs + r * kTileCells + w, srcf + (size_t)r * CF_TILE + w);
+                }
+                if constexpr (JV) {
+                    const T* srcv = vT + tile_base;
+                    for (int i = tid; i < M * CPR; i += W * 32) {
+                        const int r = i / CPR, w = (i % CPR) * PER16;
+                        cp_async16(vs + r * kTileCells + w, srcv + (size_t)r * CF_TILE + w);
+                    }
                 }
             }
             cp_async_commit();
@@ -431,7 +540,41 @@ __global__ void __launch_bounds__(W * 32, 1)
         if (tid == 0) s_next = 0;
         __syncthreads();
         const int b0 = sc.bin_begin[bin], nb = sc.bin_begin[bin + 1] - b0;
-        double* qtc = QT + tile_base + (lane & 15);
+        const bool live = !CM || cell0 + (lane & 15) < n_cells;
+        double* qtc = CM ? QT + (size_t)(live ? cell0 + (lane & 15) : 0) * M : QT + tile_base + (lane & 15);
+        if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT) {
+            if (nb < W && nb <= sc.share) {
+                // part sums [item][part][k1][lane] behind the warps' R buffers
+                double* parts = reinterpret_cast<double*>(smem) + (size_t)(JV ? 2 : 1) * M * kTileCells +
+                                (RG ? 0 : (size_t)W * WB);
+                for (;;) {
+                    int i = 0;
+                    if (lane == 0) i = atomicAdd(&s_next, 1);
+                    i = __shfl_sync(0xffffffffu, i, 0);
+                    if (i >= nb * kRowParts) break;
+                    double sum[K];
+                    pair_item<K, EXACT, JV, RG, T, CM, TS>(op, sc.items[sc.bin_item[b0 + i / kRowParts]], fs, vs, rb, qtc,
+                                                       lane, live, i % kRowParts, sum);
+#pragma unroll
+                    for (int k1 = 0; k1 < K; ++k1) parts[(i * K + k1) * 32 + lane] = sum[k1];
+                }
+                __syncthreads();
+                for (int i = warp; i < nb; i += W) {
+                    const int2 it = sc.items[sc.bin_item[b0 + i]];
+                    const int q1 = lane < 16 ? it.x : it.y;
+                    if (q1 < 0 || !live) continue;
+#pragma unroll
+                    for (int k1 = 0; k1 < K; ++k1) {
+                        double* out = qtc + q_off<K, CM>(q1, k1, op.n_q);
+                        double x = *out;
+                        for (int g = 0; g < kRowParts; ++g) x += parts[((i * kRowParts + g) * K + k1) * 32 + lane];
+                        *out = x;
+                    }
+                }
+                __syncthreads();
+                continue;
+            }
+        }
         for (;;) {
             int i = 0;
             if (lane == 0) i = atomicAdd(&s_next, 1);
@@ -440,15 +583,17 @@ __global__ void __launch_bounds__(W * 32, 1)
             if constexpr (SPLIT)
                 pair_split_item<K, T>(op, sc.items[sc.bin_item[b0 + i]], fs, rb, qtc, lane);
             else
-                pair_item<K, EXACT, JV, RG, T>(op, sc.items[sc.bin_item[b0 + i]], fs, vs, rb, qtc, lane);
+                pair_item<K, EXACT, JV, RG, T, CM, TS>(op, sc.items[sc.bin_item[b0 + i]], fs, vs, rb, qtc, lane, live);
         }
         __syncthreads();
     }
 }
 
+// sums: the warps keep row sums behind their R_t (pair_sums_shared)
 template <int K, typename T = double>
-constexpr size_t pair_smem_bytes(int M, int W, bool jv, bool rg) {
-    return sizeof(T) * ((size_t)(jv ? 2 : 1) * M * kTileCells + (rg ? 0 : (size_t)W * RPair<K, T>::SIZE));
+constexpr size_t pair_smem_bytes(int M, int W, bool jv, bool rg, bool sums = false) {
+    return sizeof(T) * ((size_t)(jv ? 2 : 1) * M * kTileCells +
+                        (rg ? 0 : (size_t)W * (RPair<K, T>::SIZE + (sums ? K * 32 : 0))));
 }
 
 }  // namespace cf

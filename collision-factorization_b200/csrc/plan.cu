@@ -56,19 +56,6 @@ int fail(int status, const char* fmt, ...) {
 
 constexpr int kMaxK = 16;
 
-// BF16 bits of a finite float, rounded to nearest even; and back
-static unsigned short bf16_bits(float x) {
-    uint32_t u;
-    std::memcpy(&u, &x, 4);
-    u += 0x7fffu + ((u >> 16) & 1u);
-    return (unsigned short)(u >> 16);
-}
-static float bf16_value(unsigned short b) {
-    const uint32_t u = (uint32_t)b << 16;
-    float x;
-    std::memcpy(&x, &u, 4);
-    return x;
-}
 constexpr int kCounterSlots = 64;  // work-queue heads per plan (one per stream in use)
 #ifndef CF_HOST_STREAMS
 #define CF_HOST_STREAMS 3
@@ -430,27 +417,19 @@ int build_plan(cf_plan* p, const double* labels, const double* vals, const doubl
     CF_TRY(upload(&p->d_e_q23, e_q23, bytes));
     CF_TRY(upload(&p->d_e_g, e_g, bytes));
     CF_TRY(upload(&p->d_R, Rv, bytes));
-    std::vector<float> R32(Rv.begin(), Rv.end());
-    CF_TRY(upload(&p->d_R32, R32, bytes));
-    if (K == 8) {
-        std::vector<double> RT(Rv.size());
-        for (int t = 0; t < p->n_l; ++t)
-            for (int k1 = 0; k1 < 8; ++k1)
-                for (int k2 = 0; k2 < 8; ++k2)
-                    for (int k3 = 0; k3 < 8; ++k3)
-                        RT[(size_t)t * 512 + k1 * 64 + 8 * k2 + k3] = Rv[(size_t)t * 512 + k1 + 8 * k2 + 64 * k3];
-        CF_TRY(upload(&p->d_RT, RT, bytes));
-        // R_t^T = hi + lo in BF16 (round to nearest even), [t][hi, lo][k1][kk]
-        std::vector<unsigned short> RTbf(2 * RT.size());
-        for (int t = 0; t < p->n_l; ++t)
-            for (int e = 0; e < 512; ++e) {
-                const double r = RT[(size_t)t * 512 + e];
-                const unsigned short hi = bf16_bits((float)r);
-                const unsigned short lo = bf16_bits((float)(r - (double)bf16_value(hi)));
-                RTbf[(size_t)t * 1024 + e] = hi;
-                RTbf[(size_t)t * 1024 + 512 + e] = lo;
-            }
-        CF_TRY(upload(&p->d_RTbf, RTbf, bytes));
+    {
+        // the other copies of R are made from it on the device
+        const size_t n = Rv.size(), n8 = K == 8 ? n : 0;
+        CF_CUDA(cudaMalloc((void**)&p->d_R32, std::max<size_t>(n, 1) * sizeof(float)));
+        if (n8) {
+            CF_CUDA(cudaMalloc((void**)&p->d_RT, n * sizeof(double)));
+            CF_CUDA(cudaMalloc((void**)&p->d_RTbf, 2 * n * sizeof(unsigned short)));
+        }
+        bytes += (int64_t)(n * sizeof(float) + n8 * (sizeof(double) + 2 * sizeof(unsigned short)));
+        if (n) {
+            cf::derive_r_kernel<<<(unsigned)((n + 255) / 256), 256>>>(p->d_R, p->d_R32, p->d_RT, p->d_RTbf, n);
+            CF_CUDA(cudaGetLastError());
+        }
     }
     CF_TRY(upload(&p->d_item_q1, items, bytes));
     CF_TRY(upload(&p->d_bin_begin, bin_begin, bytes));
@@ -465,6 +444,7 @@ int build_plan(cf_plan* p, const double* labels, const double* vals, const doubl
     CF_CUDA(cudaDeviceGetAttribute(&p->n_sms, cudaDevAttrMultiProcessorCount, dev));
     CF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     p->max_smem = (size_t)optin;
+    CF_CUDA(cudaStreamSynchronize(nullptr));  // a launch on another stream may read what the kernels here wrote
     p->dev_bytes = bytes;
     return CF_OK;
 }
@@ -502,7 +482,7 @@ int dispatch(const cf_plan* p, int what, bool exact, const double* fT, const dou
              cudaStream_t st, const float* fT32 = nullptr, bool bf16 = false, const StreamSync* ss = nullptr,
              const double* f_cm = nullptr, double* q_cm = nullptr, bool few = false,
              const double* few_host_f = nullptr, const double* few_host_q = nullptr, const float* vT32 = nullptr,
-             bool rows = false, const double* v_cm = nullptr) {
+             bool rows = false, const double* v_cm = nullptr, bool pair_cm = false) {
     const int64_t nt = n_tiles_for(B);
     // The folded operator has about half the COO entries per slice of the plain one, and its tile
     // routine groups them by q2, so its Phi step is light next to the K^3 step; there the tile kernel
@@ -521,6 +501,7 @@ int dispatch(const cf_plan* p, int what, bool exact, const double* fT, const dou
     a.vT32 = vT32;
     a.rows = rows;
     a.v_cm = v_cm;
+    a.pair_cm = pair_cm;
     cf::LaunchResult r{8, 0, cudaSuccess};
     switch (p->k) {
 #define CF_K(KK) \
@@ -542,6 +523,13 @@ int dispatch(const cf_plan* p, int what, bool exact, const double* fT, const dou
         return fail(CF_EUNSUPPORTED, "form or kernel path not built for K = %d ("
                     "the tile-resident kernels need an even K <= 8 and a tile that fits in shared memory)", p->k);
     if (r.status != CF_OK) return fail(r.status, "launch failed for K = %d", p->k);
+    return CF_OK;
+}
+
+// The batch limit of the layout passes, which holds for the forms that used to need them too.
+int check_tiles(int64_t B) {
+    if (n_tiles_for(B) > 65535)
+        return fail(CF_ESHAPE, "B = %lld exceeds %d cells per call", (long long)B, 65535 * CF_TILE);
     return CF_OK;
 }
 
@@ -668,6 +656,18 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
             return dispatch(target, 0, false, nullptr, nullptr, nullptr, B, st, nullptr, false, &resident, f_dev,
                             q_dev);
         }
+    }
+    // The fast FP64 forms that the automatic order gives to the pair kernel: one launch on the cell-major
+    // arrays, without the layout passes (three or four launches of 2-5 us each).  A batch within one
+    // half-tile keeps the passes.
+    if (!exact && f32 == 0 && (what == 0 || what == 2) && B > 16 &&
+        (p->path == cf::PATH_PAIR || (p->path == cf::PATH_AUTO && !(sym && p->k % 2 == 0))) &&
+        cf::pair_fits(p->n_q, p->k, what == 2, p->max_smem)) {
+        cf_plan* target = p;
+        if (sym) CF_TRY(get_sym(p, &target));
+        CF_TRY(check_tiles(B));
+        return dispatch(target, what, false, nullptr, nullptr, nullptr, B, st, nullptr, false, nullptr, f_dev, q_dev,
+                        false, nullptr, nullptr, nullptr, false, what == 2 ? v_dev : nullptr, true);
     }
     float* vT32 = (f32 && what == 2) ? reinterpret_cast<float*>(vT) : nullptr;  // FP32 J.v: v's FP32 tiles
     if (f32)

@@ -32,6 +32,34 @@ struct TileSched {
     int* counter;          // zeroed before the launch
 };
 
+// Units of a persistent launch: whole tiles, then tiles cut into 4 row bins, then the last into 16, so that the
+// CTAs end within a sixteenth of a tile's work of one another.
+struct UnitCuts {
+    int n_whole, n_four;  // tiles taken whole; the end of those cut into 4
+    int n_units;
+};
+__host__ __device__ inline void unit_of(const UnitCuts& c, int u, int& tile, int& bin) {
+    const int fours = (c.n_four - c.n_whole) * 4;
+    if (u < c.n_whole) {
+        tile = u;
+        bin = 0;
+    } else if (u < c.n_whole + fours) {
+        tile = c.n_whole + (u - c.n_whole) / 4;
+        bin = 1 + (u - c.n_whole) % 4;
+    } else {
+        tile = c.n_four + (u - c.n_whole - fours) / 16;
+        bin = 5 + (u - c.n_whole - fours) % 16;
+    }
+}
+// Up to a whole tile per CTA in quarters; with `fine` (a sixteenth still occupies a CTA's warps) an eighth of a tile
+// per CTA in sixteenths after them; everything in sixteenths where quarters would not go round once.
+inline UnitCuts cut_units(int64_t n_tiles, int64_t ctas, bool fine) {
+    const int64_t n16 = n_tiles * 4 < ctas ? n_tiles : !fine ? 0 : (n_tiles < ctas / 8 ? n_tiles : ctas / 8);
+    const int64_t n4 = n_tiles - n16 < ctas ? n_tiles - n16 : ctas;
+    const int64_t n_whole = n_tiles - n16 - n4;
+    return {(int)n_whole, (int)(n_whole + n4), (int)(n_whole + n4 * 4 + n16 * 16)};
+}
+
 __host__ __device__ constexpr int bin_base(int split) { return split == 4 ? 1 : 5; }
 
 template <int K>
@@ -44,6 +72,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
@@ -52,6 +84,22 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 template <int K, bool CELL_MAJOR>
 __device__ __forceinline__ size_t q_off(int q1, int k1, int n_q) {
     return CELL_MAJOR ? (size_t)q1 + (size_t)k1 * n_q : (size_t)(q1 * K + k1) * CF_TILE;
+}
+
+// Stage a half-tile from the caller's cell-major array: element j = q + N_Q k of cell c goes to row q K + k;
+// a warp reads two consecutive j of 16 cells and writes two 16-cell rows of shared memory.
+template <int K>
+__device__ __forceinline__ void stage_cells(double* fs, const double* __restrict__ f, int n_q, long long cell0,
+                                            long long n_cells, int tid, int threads) {
+    const int M = n_q * K;
+    for (int i = tid; i < M * kTileCells; i += threads) {
+        const int c = i & 15, j = i >> 4;
+        const int r = (j % n_q) * K + j / n_q;
+        if (cell0 + c < n_cells)
+            cp_async8(fs + r * kTileCells + c, f + (size_t)(cell0 + c) * M + j);
+        else
+            fs[r * kTileCells + c] = 0.0;
+    }
 }
 
 // Contract every slice of one q1 for the resident half-tile.  qtc points at this lane's cell of
@@ -553,11 +601,6 @@ constexpr size_t tile4_smem_bytes(int M, int W, bool jv) {
 // epoch into host_done[c], a word of mapped pinned host memory the host polls before queueing the
 // chunk's download.
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-
 __device__ __forceinline__ int ld_acquire(const int* p) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
@@ -607,16 +650,7 @@ __global__ void __launch_bounds__(W * 32, 1)
                 }
             }
             __syncthreads();
-            // element j = q + N_Q k of cell c (cell-major) goes to row q K + k of the tile; a warp
-            // reads two consecutive j of 16 cells and writes two 16-cell rows of shared memory
-            for (int i = tid; i < M * kTileCells; i += W * 32) {
-                const int c = i & 15, j = i >> 4;
-                const int r = (j % op.n_q) * K + j / op.n_q;
-                if (cell0 + c < n_cells)
-                    cp_async8(fs + r * kTileCells + c, f + (size_t)(cell0 + c) * M + j);
-                else
-                    fs[r * kTileCells + c] = 0.0;
-            }
+            stage_cells<K>(fs, f, op.n_q, cell0, n_cells, tid, W * 32);
             cp_async_commit();
             cp_async_wait_all();
             staged = ht;

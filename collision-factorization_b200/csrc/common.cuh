@@ -33,6 +33,12 @@ struct DevOp {
     const float* R32;  // FP32 copy of R for the FP32 form
     const double* RT;  // K = 8 only: R_t transposed to [k1][kk = K k2 + k3] (A operands of the MMA kernel)
     const unsigned short* RTbf;  // K = 8 only: R_t^T split in BF16, [t][hi, lo][k1][kk] (BF16-split form)
+    // outer-product kernels (K <= 8): per slice (t, first chunk, chunks with a second q3, chunks); per chunk
+    // 4 x (q2, q3a, q3b) and 4 x G of both; R_t in lane order (null where the plan has no such tables)
+    const int* x_q1;  // [N_Q + 1] x_slice range of each q1
+    const int4* x_slice;
+    const unsigned char* x_chunk;
+    const double2* x_R;
     const int* item_q1;
     int grouped;  // each slice's entries sorted by q2 (the folded operator); bit 0: the fast Q tile
                   // routine sums G f(q3) over each run of equal q2 before one outer product with

@@ -97,6 +97,48 @@ constexpr bool pair_fits(int n_q, int K, bool jv, size_t max_smem) {
     return K <= 8 && sizeof(double) * ((size_t)(jv ? 2 : 1) * n_q * K * 16 + (size_t)pair_W(K, jv) * pair_warp_doubles(K, jv)) +
                              256 <= max_smem;
 }
+// K that the outer-product kernels (outer_kernels.cuh) take.
+constexpr bool outer_for(int K) { return K >= 7 && K <= 8; }
+
+// Where they are the faster family (B200, us, outer / tile or pair): from L = 7 on, at every batch (folded Q, K = 8: L = 10,
+// 4096 cells 1542 / 1642, L = 13, 1000 cells 1122 / 1928; J.v, L = 10: 2193 / 3060); below, for batches of at most half
+// an SM's half-tile each (L = 5, 300 cells: 45 / 59; 4096 cells: 205 / 191), whose rows their teams spread better;
+// and the plain K = 8 forms always (L = 5, 4096 cells: 305 / 335).
+constexpr bool outer_takes(int n_q, int K, bool folded, int64_t n_cells, int n_sms) {
+    return outer_for(K) && (n_q >= 64 || (K == 8 && !folded) || (n_cells + 15) / 16 * 2 <= n_sms);
+}
+
+// Shared-memory geometry of the outer-product kernels.  Cells lie in pairs, [pair][k][q][cell of the pair],
+// with rows of NQP doubles per cell fixed at compile time (one of two widths, 4 modulo 8, so that the 8 lanes
+// of a 128-bit load phase, 2 k x 4 q distinct modulo 4, hit distinct banks) and an odd pair stride.
+constexpr int outer_nqp(int width) { return width == 0 ? 132 : 268; }  // L <= 10, L <= 15
+constexpr int outer_pair(int K, int nqp) { return K * nqp + 1; }       // 16-byte elements per pair of cells
+constexpr int kOuterCells = 4;   // cells per warp: 128 registers a lane hold acc and Phi, 16 warps fit
+constexpr int kOuterWarps = 16;
+constexpr int kOuterChunks = 8;  // chunks of 4 runs per slice at most (longer slices are cut)
+// A team's ring of two packets of up to outer_group() slices: R_t in lane order, the chunks, the heads.  Q takes
+// two slices to a packet at the narrow width (half the team barriers: 1552 against 1591 us at L = 10, K = 8,
+// 4096 cells); with f and v resident, or the wide rows, only one fits.
+constexpr int outer_group(int nqp, bool jv) { return !jv && nqp == outer_nqp(0) ? 2 : 1; }
+constexpr int outer_ring_bytes(int K, int nqp, bool jv) {
+    return 2 * outer_group(nqp, jv) * (K * 512 + kOuterChunks * 96 + 32) + 32;
+}
+// nc cells of f (and v), a ring per team of nc / 4 warps, and a task per q1 row.
+constexpr size_t outer_smem_bytes(int n_q, int K, int nqp, int nc, bool jv) {
+    return (size_t)(jv ? 2 : 1) * (nc / 2) * outer_pair(K, nqp) * 16 +
+           (size_t)(kOuterWarps * kOuterCells / nc) * outer_ring_bytes(K, nqp, jv) + (size_t)n_q * 48;
+}
+// The widest unit that fits: 16 cells per unit before 8; (width, cells), or cells = 0 where none does.
+struct OuterFit {
+    int width, nc;
+};
+constexpr OuterFit outer_fit(int n_q, int K, bool jv, size_t max_smem) {
+    const int width = n_q <= outer_nqp(0) ? 0 : 1;
+    if (n_q > outer_nqp(width)) return {0, 0};
+    for (int nc = 16; nc >= 8; nc -= 8)
+        if (outer_smem_bytes(n_q, K, outer_nqp(width), nc, jv) + 256 <= max_smem) return {width, nc};
+    return {0, 0};
+}
 constexpr int jv_P(int K) { return K <= 6 ? 1 : (K <= 8 ? 2 : 4); }
 
 }  // namespace cf

@@ -80,6 +80,18 @@ static __global__ void __launch_bounds__(256) derive_r_kernel(const double* __re
     RTbf[t * 1024 + 512 + j] = bf16_round((float)(r - (double)__uint_as_float((uint32_t)hi << 16)));
 }
 
+// R_t in the lane order of the outer-product kernels: dst[(t K + k1) 32 + lane] = R_t[k1][k2 = lane / 4][k3 = 2 (lane % 4),
+// + 1], zero where k2 or k3 is past K.
+static __global__ void __launch_bounds__(256) lane_order_kernel(const double* __restrict__ R, double2* __restrict__ dst,
+                                                                size_t n, int K) {
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int lane = (int)(i % 32), k2 = lane >> 2, k3 = 2 * (lane & 3);
+    const size_t tk = i / 32, t = tk / K, k1 = tk % K;
+    const double* src = R + t * K * K * K + k1 + (size_t)K * k2 + (size_t)K * K * k3;
+    dst[i] = make_double2(k2 < K && k3 < K ? src[0] : 0.0, k2 < K && k3 + 1 < K ? src[(size_t)K * K] : 0.0);
+}
+
 // FP64 FMA throughput probe: kProbeChains independent DFMA chains per thread.
 constexpr int kProbeChains = 8;
 static __global__ void __launch_bounds__(256) fp64_fma_probe_kernel(double* sink, int iters, double a) {

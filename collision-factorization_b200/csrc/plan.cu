@@ -102,6 +102,10 @@ struct cf_plan {
     float* d_R32 = nullptr;  // FP32 copy of R for CF_FORM_AF_F32
     double* d_RT = nullptr;  // K = 8: R_t as [k1][8 k2 + k3] for the MMA kernel
     unsigned short* d_RTbf = nullptr;  // K = 8: the same split into BF16 hi and lo parts
+    int* d_x_q1 = nullptr;
+    int4* d_x_slice = nullptr;  // outer-product kernels' tables (build_outer)
+    unsigned char* d_x_chunk = nullptr;
+    double2* d_x_R = nullptr;
     int* d_item_q1 = nullptr;
     int* d_bin_begin = nullptr;  // q1 bins of the tile kernel's work units (bin 0 = all, 1..4, 5..20)
     int* d_bin_q1 = nullptr;
@@ -170,6 +174,10 @@ struct cf_plan {
         o.R32 = d_R32;
         o.RT = d_RT;
         o.RTbf = d_RTbf;
+        o.x_q1 = d_x_q1;
+        o.x_slice = d_x_slice;
+        o.x_chunk = d_x_chunk;
+        o.x_R = d_x_R;
         o.item_q1 = d_item_q1;
         o.grouped = grouped;
         o.n_items = n_items;
@@ -268,6 +276,10 @@ void free_plan_memory(cf_plan* p) {
     cudaFree(p->d_R32);
     cudaFree(p->d_RT);
     cudaFree(p->d_RTbf);
+    cudaFree(p->d_x_q1);
+    cudaFree(p->d_x_slice);
+    cudaFree(p->d_x_chunk);
+    cudaFree(p->d_x_R);
     cudaFree(p->d_item_q1);
     cudaFree(p->d_bin_begin);
     cudaFree(p->d_bin_q1);
@@ -288,6 +300,115 @@ void free_plan_memory(cf_plan* p) {
         if (ev) cudaEventDestroy(ev);
     for (cudaStream_t& hs : p->xs)
         if (hs) cudaStreamDestroy(hs);
+}
+
+// Tables of the outer-product kernels (outer_kernels.cuh): every slice's entries as runs of equal q2 of one
+// or two entries, four runs to a chunk, the runs of two first.  Runs of a chunk are picked so that
+// their q2, and their q3 of either column, are distinct modulo 4 as far as a few candidates allow (the
+// operands of eight lanes then lie in distinct banks: 20 % above the conflict-free count at L = 10, 39 %
+// in the list's own order).
+int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<int>& slice_t,
+                const std::vector<int>& slice_e, const std::vector<uint32_t>& e_q23, const std::vector<double>& e_g,
+                int64_t& bytes) {
+    constexpr size_t kLook = 6;  // candidates per place
+    struct Run {
+        unsigned short q2, qa, qb, two;
+        double ga, gb;
+    };
+    struct Chunk {
+        ushort4 q[4];
+        double2 g[4];
+    };
+    static_assert(sizeof(Chunk) == 96, "the kernels copy chunks of 96 bytes");
+    const size_t S = slice_t.size();
+    std::vector<int4> xs;
+    std::vector<int> xbegin(S + 1, 0), xq1(q1_begin.size());
+    std::vector<unsigned char> xb;
+    xs.reserve(S + S / 8);
+    xb.reserve((e_q23.size() / 3 + S) * sizeof(Chunk));
+    std::vector<uint64_t> ent;  // q2 << 32 | entry
+    std::vector<Run> all, one;
+    size_t n_chunks = 0;
+    for (size_t s = 0; s < S; ++s) {
+        ent.clear();
+        bool sorted = true;
+        for (int e = slice_e[s]; e < slice_e[s + 1]; ++e) {
+            const uint64_t x = (uint64_t)(e_q23[e] & 0xffffu) << 32 | (uint64_t)e;
+            sorted = sorted && (ent.empty() || ent.back() < x);
+            ent.push_back(x);
+        }
+        if (!sorted) std::sort(ent.begin(), ent.end());
+        all.clear();
+        one.clear();
+        for (size_t i = 0; i < ent.size();) {
+            const bool two = i + 1 < ent.size() && ent[i + 1] >> 32 == ent[i] >> 32;
+            const uint32_t ea = (uint32_t)ent[i], eb = two ? (uint32_t)ent[i + 1] : ea;
+            (two ? all : one).push_back({(unsigned short)(ent[i] >> 32), (unsigned short)(e_q23[ea] >> 16),
+                                         (unsigned short)(e_q23[eb] >> 16), two, e_g[ea], two ? e_g[eb] : 0.0});
+            i += two ? 2 : 1;
+        }
+        const size_t n_two = all.size();
+        all.insert(all.end(), one.begin(), one.end());
+        const int begin = (int)n_chunks;
+        for (size_t i0 = 0; i0 < all.size(); i0 += 4) {
+            int used[3][4] = {};  // residues taken in this chunk: q2, q3a, q3b
+            for (size_t i = i0; i < std::min(i0 + 4, all.size()); ++i) {
+                const size_t hi = std::min(i + kLook, i < n_two ? n_two : all.size());  // runs of two stay in front
+                size_t best = i;
+                bool flip = false;
+                int c_best = 1 << 20;
+                for (size_t c = i; c < hi && c_best > 0; ++c) {
+                    const Run& r = all[c];
+                    const int c2 = used[0][r.q2 & 3], a0 = used[1][r.qa & 3] + used[2][r.qb & 3],
+                              a1 = used[1][r.qb & 3] + used[2][r.qa & 3];
+                    if (c2 + std::min(a0, a1) < c_best) {
+                        c_best = c2 + std::min(a0, a1);
+                        best = c;
+                        flip = r.two && a1 < a0;
+                    }
+                }
+                if (best != i) std::swap(all[i], all[best]);
+                Run& r = all[i];
+                if (flip) {
+                    std::swap(r.qa, r.qb);
+                    std::swap(r.ga, r.gb);
+                }
+                ++used[0][r.q2 & 3];
+                ++used[1][r.qa & 3];
+                ++used[2][r.qb & 3];
+            }
+            Chunk c;
+            for (size_t i = 0; i < 4; ++i) {
+                // an empty slot repeats the chunk's first run with G = 0
+                const bool in = i0 + i < all.size();
+                const Run& r = all[in ? i0 + i : i0];
+                // as byte offsets in a row of cell pairs (N_Q <= 268 where the kernels run)
+                c.q[i] = make_ushort4((unsigned short)(16 * r.q2), (unsigned short)(16 * r.qa),
+                                      (unsigned short)(16 * r.qb), 0);
+                c.g[i] = in ? make_double2(r.ga, r.gb) : make_double2(0.0, 0.0);
+            }
+            xb.insert(xb.end(), (const unsigned char*)&c, (const unsigned char*)(&c + 1));
+            ++n_chunks;
+        }
+        // a ring stage holds kOuterChunks chunks; the K^3 step is linear, so a longer slice is several
+        const int n = (int)((all.size() + 3) / 4), n2 = (int)((n_two + 3) / 4);
+        for (int c = 0; c < n; c += cf::kOuterChunks)
+            xs.push_back(make_int4(slice_t[s], begin + c, std::max(0, std::min(cf::kOuterChunks, n2 - c)),
+                                   std::min(cf::kOuterChunks, n - c)));
+        xbegin[s + 1] = (int)xs.size();
+    }
+    for (size_t q = 0; q < q1_begin.size(); ++q) xq1[q] = xbegin[q1_begin[q]];
+    CF_TRY(upload(&p->d_x_q1, xq1, bytes));
+    CF_TRY(upload(&p->d_x_slice, xs, bytes));
+    CF_TRY(upload(&p->d_x_chunk, xb, bytes));
+    const size_t nR = (size_t)p->n_l * p->k * 32;
+    CF_CUDA(cudaMalloc((void**)&p->d_x_R, std::max<size_t>(nR, 1) * sizeof(double2)));
+    bytes += (int64_t)(nR * sizeof(double2));
+    if (nR > 0) {
+        cf::lane_order_kernel<<<(unsigned)((nR + 255) / 256), 256>>>(p->d_R, p->d_x_R, nR, p->k);
+        CF_CUDA(cudaGetLastError());
+    }
+    return CF_OK;
 }
 
 // Build the q1-grouped run structure (host) and upload it.
@@ -444,6 +565,8 @@ int build_plan(cf_plan* p, const double* labels, const double* vals, const doubl
     CF_CUDA(cudaDeviceGetAttribute(&p->n_sms, cudaDevAttrMultiProcessorCount, dev));
     CF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     p->max_smem = (size_t)optin;
+    if (cf::outer_for(K) && cf::outer_fit(NQ, K, false, p->max_smem).nc > 0)
+        CF_TRY(build_outer(p, q1_begin, slice_t, slice_e, e_q23, e_g, bytes));
     CF_CUDA(cudaStreamSynchronize(nullptr));  // a launch on another stream may read what the kernels here wrote
     p->dev_bytes = bytes;
     return CF_OK;
@@ -630,6 +753,17 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
     const size_t tb = tiled_bytes(p, B);
     const size_t need = tb * (what == 2 ? 3 : 2);
     if (ws_bytes < need) return fail(CF_EINVAL, "workspace of %zu bytes is smaller than %zu", ws_bytes, need);
+    // The fast FP64 Q and J.v forms on the outer-product kernel: one launch on the cell-major arrays.
+    if (!exact && f32 == 0 && (what == 0 || what == 2) && p->path == cf::PATH_AUTO &&
+        cf::outer_takes(p->n_q, p->k, sym, B, p->n_sms) &&
+        cf::outer_fit(p->n_q, p->k, what == 2, p->max_smem).nc > 0) {
+        cf_plan* target = p;
+        if (sym) CF_TRY(get_sym(p, &target));
+        if (!streamable(p, target, what, exact, f32)) CF_TRY(check_tiles(B));
+        const StreamSync resident{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, 0};
+        return dispatch(target, what, false, nullptr, nullptr, nullptr, B, st, nullptr, false, &resident, f_dev, q_dev,
+                        false, nullptr, nullptr, nullptr, false, what == 2 ? v_dev : nullptr);
+    }
     double* fT = (double*)ws;
     double* QT = (double*)((char*)ws + tb);
     double* vT = what == 2 ? (double*)((char*)ws + 2 * tb) : nullptr;

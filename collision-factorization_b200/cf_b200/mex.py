@@ -11,17 +11,13 @@ Here the work runs on the GPU through libcf_b200.so.  Unlike the reference, bad 
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import numpy as np
 
 from . import _lib
 
-_D = C.POINTER(C.c_double)
 
-
-def _ptr(a: np.ndarray):
-    return a.ctypes.data_as(_D)
+def _ptr(a: np.ndarray) -> int:
+    return a.ctypes.data  # the caller keeps `a`
 
 
 def _in(a) -> np.ndarray:

@@ -72,3 +72,21 @@ struct StreamSync {
 // Lanes per cell used by the angular-first kernels: the K x K Phi accumulator of one cell
 // is split over P lanes (by k3 column) once it no longer fits one lane's registers.
 __host__ __device__ constexpr int af_lanes_per_cell(int K) { return K <= 8 ? 1 : (K <= 12 ? 2 : 4); }
+
+// cp.async: 16 bytes (through L2 only) or 8 bytes from global into shared memory.
+namespace cf {
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { cp_async_wait<0>(); }
+}  // namespace cf

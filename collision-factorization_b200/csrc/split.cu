@@ -121,23 +121,24 @@ struct SplitArgs {
     int n_q, L;
     int tseg;                  // t per accumulation segment (int32 bound)
     int n_abuf;                // A buffers of six planes each (2 where shared memory allows, else 1)
-    // the l-block kernel: f packed per cell group as [q][k][cell], one stage per l-triplet
-    const double* pf;          // [n_cg][N_Q][K][C]
+    // the l-block kernels: f packed per cell group, one stage per l-triplet
+    const uint4* recs;         // run records (LbRun), item after item
+    const double* pf;          // [n_cg][N_Q] rows of K C values (pack_cg_kernel)
     const int* t_l23;          // per l-triplet: l2 | l3 << 8
     int n_ring, stage_bytes;   // stages in the ring, bytes per stage (R_t first, then the f rows)
-    const int4* items;         // per band, its (t, row) slices in t-major order (lbi_*)
+    const int4* items;         // per band, its (t, row) slices in t-major order (LBI_*)
     const int* t_items;        // per t-list position of a band: its number of items
     int max_rows, max_t;       // sizes of the per-CTA row and t tables
     long long wait_cycles;     // the l-block kernel's budget per bounded wait (SM clocks)
     int no_copy;               // self-test: no stage is ever filled, so every wait runs out
     // shared-memory offsets (bytes)
-    int off_a, off_b, off_f, off_mb, off_red, off_scale, off_eexp, off_bar, off_misc;
+    int off_a, off_b, off_f, off_mb, off_red, off_scale, off_eexp, off_bar, off_misc, off_rec;
 };
 
 enum { U_L1 = 0, U_R0, U_NR, U_S, U_TLOFF, U_NT, U_TABOFF, U_BROWS, U_REM, U_INTS };
 
 struct Layout {
-    int off_a, off_b, off_f, off_mb, off_red, off_scale, off_eexp, off_bar, off_misc, total;
+    int off_a, off_b, off_f, off_mb, off_red, off_scale, off_eexp, off_bar, off_misc, off_rec, total;
 };
 
 template <int K, int C>
@@ -193,13 +194,15 @@ Layout band64_layout(int n_q, int warps) {
 constexpr int kLbCells = 8;
 constexpr int kLbWarps = 16;
 constexpr int kLbMaxRing = 8;
+constexpr int kLbRecs = 16;  // runs per record buffer: a slice of the largest operators has 14 on average
 
 __host__ __device__ constexpr bool lblock_supported_k(int k) { return k == 8 || k == 12; }
 
 // The l-block kernel's shared memory: the ring of stages (R_t as the kernel reads it, then at most
 // max_rows packed f rows of K x cells values each), the band's FP64 Q rows of the CTA's cells, and the
-// counter, done words, row tickets, per-t item totals and stage assignments.
-inline Layout lblock_layout(int n_ring, int stage_bytes, int k, int max_rows, int max_t, int cells) {
+// counter, done words, row tickets, per-t item totals and stage assignments, and per warp two buffers
+// of kLbRecs run records.
+inline Layout lblock_layout(int n_ring, int stage_bytes, int k, int max_rows, int max_t, int cells, int rec_bytes) {
     Layout l{};
     int o = 0;
     auto take = [&](int bytes, int align) {
@@ -212,6 +215,7 @@ inline Layout lblock_layout(int n_ring, int stage_bytes, int k, int max_rows, in
     l.off_red = take(max_rows * k * cells * (int)sizeof(double), 16);
     l.off_bar = take(16 * (int)sizeof(uint64_t), 16);
     l.off_misc = take((2 + 2 * kLbMaxRing + max_rows + max_t) * (int)sizeof(int), 16);
+    l.off_rec = take(kLbWarps * 2 * kLbRecs * rec_bytes, 16);
     l.total = o;
     return l;
 }
@@ -787,8 +791,8 @@ __global__ void __launch_bounds__(W * 32, 1) af_band64_kernel(SplitArgs a) {
 // at most 4L rows of the cell's N_Q = (L+1)^2.  So instead of holding all of f for 4 cells (which is
 // what fits at L = 16, K = 12: 27.7 KB of FP64 f per cell), a CTA holds C = 8 cells and stages, per
 // t of its band's t-list, R_t and those two row blocks into a ring of shared-memory stages: three
-// cp.async.bulk copies per stage on one mbarrier (transaction bytes), from f packed per cell group as
-// [q][k][cell] so that a band's rows are one contiguous run.  Every COO entry's index work and every
+// cp.async.bulk copies per stage on one mbarrier (transaction bytes), from f packed per cell group
+// (q outermost) so that a band's rows are one contiguous run.  Every COO entry's index work and every
 // R_t load then serves 8 cells instead of 4.
 //
 // One CTA takes one (l1 band, 8-cell group).  A band's rows do not divide evenly over the warps of a
@@ -799,8 +803,16 @@ __global__ void __launch_bounds__(W * 32, 1) af_band64_kernel(SplitArgs a) {
 // in t order (a ticket per row: the warp holding the row's slice number ord waits until ord - 1 has
 // been added), so the sums, and the bits of Q, do not depend on which warp ran which item.  The stage
 // of t-list position ti is refilled with ti + n_ring by the warp that finishes the last item of ti.
+//
+// A slice comes as run records (LbRun) that each warp copies (cp.async) into its own two shared-memory
+// buffers, one item ahead, so neither the index work of the entries nor their latency is in the Phi loop.
+// At L = 16, K = 12, 1024 cells, against one entry at a time through shuffles: FP64 6.90 -> 6.08 ms,
+// FP32 (with the packed multiply-add) 4.37 -> 3.33 ms, both with the same bits.  What bounds them now is
+// shared-memory bandwidth: an item (14 runs on average) reads 14 x 40 + 144 wavefronts in FP64 (f, the
+// records; the R_t fragments), 71 % of the time at one per clock, beside 582 clocks of the FP64 pipe; in
+// FP32 14 x 26 + 460, 76 %.
 
-// f cell-major [B][K][N_Q] -> packed [cg][q][k][C], or with CELLROWS [cg][q][C][k] (zero past the
+// f cell-major [B][K][N_Q] -> packed [cg][q][k / 2][C][k % 2], or with CELLROWS [cg][q][C][k] (zero past the
 // end of the batch).  One CTA per
 // (cell group, 32 rows q), in a one-dimensional grid: the C cells' K x 32 block is read along q
 // (coalesced) into shared memory and written out as one contiguous run.
@@ -819,90 +831,44 @@ __global__ void __launch_bounds__(256) pack_cg_kernel(const double* __restrict__
         const long long cell = cg * C + c;
         double v = 0.0;
         if (qq < nq && cell < n_cells) v = __ldg(f + cell * M + (long long)k * n_q + q0 + qq);
-        tile[CELLROWS ? (qq * C + c) * K + k : (qq * K + k) * C + c] = (T)v;
+        tile[CELLROWS ? (qq * C + c) * K + k : (qq * K + (k & ~1)) * C + 2 * c + (k & 1)] = (T)v;
     }
     __syncthreads();
     T* out = pf + (cg * n_q + q0) * K * C;
     for (int i = threadIdx.x; i < nq * K * C; i += blockDim.x) out[i] = tile[i];
 }
 
-// The lane layout of the l-block kernels: C cells per CTA, P = 32 / C lanes (parts) per cell, each
-// holding all K values of k2 and KQ = K / P values of k3 of the cell's Phi.  FP64 (C = 8): part p
-// owns k3 = p KQ .. p KQ + KQ - 1 (the packed rows k3 of the four parts fall on distinct banks);
-// FP32 (C = 16): part p owns k3 = p, p + 2, ... (blocked halves would put both half-warps' 32-bit
-// loads on the same 16 banks).  R_t per stage is [part][e = k2 KQ + y][k1] in T, 16 bytes of padding
-// after each part.
-template <int K, int C, typename T>
+// The lane layout of the FP32 l-block kernel: C = 16 cells per CTA, P = 2 lanes (parts) per cell, each
+// holding all K values of k2 and the KQ = K / 2 values k3 = p, p + 2, ... of part p of the cell's Phi, as
+// pairs (k2, k2 + 1) for the packed FP32 multiply-add (fma.rn.f32x2, two products per instruction: the
+// kernel is bound by instruction issue and shared-memory reads).  f is staged as [q][k / 2][cell][k % 2]:
+// a pair of k2 is one 8-byte load, and the two parts' k3 are the two halves of the cells' pairs.  R_t per
+// stage is [part][k2][y][k1], 16 bytes of padding after each part: 16 bytes hold two pairs of k1, which
+// multiply one Phi value given twice, so every k1 sums its products one by one in the order of (k2, y).
+template <int K>
 struct LbShape {
+    static constexpr int C = 2 * kLbCells;
     static constexpr int P = 32 / C;
-    static constexpr int KH = K;
     static constexpr int KQ = K / P;
-    static constexpr int E = KH * KQ;
-    static constexpr int PS = E * K + 16 / (int)sizeof(T);  // T words per part
-    static constexpr int RT_BYTES = P * PS * (int)sizeof(T);
-    static constexpr bool INTERLEAVED = sizeof(T) == 4;
-    __host__ __device__ static constexpr int k3_base(int p) { return INTERLEAVED ? p : p * KQ; }
-    static constexpr int K3_STEP = INTERLEAVED ? P : 1;
-    __host__ __device__ static constexpr int k3(int p, int y) { return k3_base(p) + y * K3_STEP; }
+    static constexpr int PS = K * KQ * K + 4;  // floats per part
+    static constexpr int RT_BYTES = P * PS * (int)sizeof(float);
+    __host__ __device__ static constexpr int r_at(int part, int k1, int k2, int y) {
+        return part * PS + (k2 * KQ + y) * K + k1;
+    }
 };
 
-// Phi of one slot on a stage: rows of the stage are local (q2 - b2, q3 - b3), f at
-// fsg[(row K + k) C + cell]; grouped by q2 as slot_phi.
-template <int K, int C, typename T>
-__device__ __forceinline__ void slot_phi_staged(const double* __restrict__ gv, const uint32_t* __restrict__ eq23,
-                                                const T* __restrict__ fsg, const SlotEntries& se, int lane,
-                                                int c, int part, int b2, int b3,
-                                                T (&phi)[LbShape<K, C, T>::KH][LbShape<K, C, T>::KQ]) {
-    using S = LbShape<K, C, T>;
-    constexpr int KH = S::KH, KQ = S::KQ;
-    const int k3o = S::k3_base(part);
-#pragma unroll
-    for (int x = 0; x < KH; ++x)
-#pragma unroll
-        for (int y = 0; y < KQ; ++y) phi[x][y] = (T)0;
-    const int cb = se.cb, ce = se.ce;
-    if (cb >= ce) return;
-    T h[KQ];
-#pragma unroll
-    for (int y = 0; y < KQ; ++y) h[y] = (T)0;
-    int cur = -1;
-    auto flush = [&]() {
-        const T* __restrict__ f2p = fsg + (size_t)cur * K * C + c;
-#pragma unroll
-        for (int x = 0; x < KH; ++x) {
-            const T f2 = f2p[x * C];
-#pragma unroll
-            for (int y = 0; y < KQ; ++y) phi[x][y] = fma(f2, h[y], phi[x][y]);
-        }
-#pragma unroll
-        for (int y = 0; y < KQ; ++y) h[y] = (T)0;
-    };
-    for (int eb = cb; eb < ce; eb += 32) {
-        const int nb = min(32, ce - eb);
-        uint32_t my_q23 = se.q23;
-        double my_g = se.g;
-        if (eb != cb) {
-            my_q23 = 0;
-            my_g = 0.0;
-            if (lane < nb) {
-                my_q23 = __ldg(eq23 + eb + lane);
-                my_g = __ldg(gv + eb + lane);
-            }
-        }
-        for (int j = 0; j < nb; ++j) {
-            const uint32_t q23 = __shfl_sync(0xffffffffu, my_q23, j);
-            const T g = (T)__shfl_sync(0xffffffffu, my_g, j);
-            const int q2 = (int)(q23 & 0xffffu) - b2, q3 = (int)(q23 >> 16) - b3;
-            if (q2 != cur) {
-                if (cur >= 0) flush();
-                cur = q2;
-            }
-            const T* __restrict__ f3p = fsg + ((size_t)q3 * K + k3o) * C + c;
-#pragma unroll
-            for (int y = 0; y < KQ; ++y) h[y] = fma(g, f3p[y * S::K3_STEP * C], h[y]);
-        }
-    }
-    if (cur >= 0) flush();
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void ffma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
 // The FP64 l-block kernel's K^3 step on the FP64 tensor cores (warp-level mma.sync m8n8k4; B200's
@@ -923,26 +889,62 @@ struct LbMma {
     static constexpr int RT_BYTES = MT * S * 32 * 8;  // A fragments of one R_t
 };
 
-// Phi of one item on an FP64 cell-rows stage (f at fsg[(row C + cell) K + k], rows local as in
-// slot_phi_staged), for lane (cell c, part p): phi[k2][y], k3 = p KQ + y; grouped by q2.
+// The Phi step reads run records: up to two entries (q2, q3a, G a), (q2, q3b, G b) of a slice with the
+// same q2 (the selection rules allow two m3 per (m1, m2); a longer run takes several records), a missing
+// second entry as G b = 0 on q3a.  The rows' offsets in the stage are in bytes, so a run costs no index
+// arithmetic, and both kernels read run i + 1 while they multiply run i.  FP64: 32 bytes {Ga, Gb, off2,
+// off3a, off3b, -}; FP32: 16 bytes {Ga, Gb, off2, off3a / 16 | off3b / 16 << 16}.
+template <typename T>
+struct LbRun {
+    static constexpr int BYTES = sizeof(T) == 8 ? 32 : 16;
+    T ga, gb;
+    uint32_t off2, off3a, off3b;
+    __device__ __forceinline__ void read(const unsigned char* p) {
+        if constexpr (sizeof(T) == 8) {
+            const double2 g = *reinterpret_cast<const double2*>(p);
+            const uint4 o = *reinterpret_cast<const uint4*>(p + 16);
+            ga = g.x;
+            gb = g.y;
+            off2 = o.x;
+            off3a = o.y;
+            off3b = o.z;
+        } else {
+            const uint4 o = *reinterpret_cast<const uint4*>(p);
+            ga = __uint_as_float(o.x);
+            gb = __uint_as_float(o.y);
+            off2 = o.z;
+            off3a = (o.w & 0xffffu) << 4;
+            off3b = (o.w >> 16) << 4;
+        }
+    }
+};
+
+// phi += the n runs at rec, FP64: lane (cell c, part p) holds phi[k2][y], k3 = p KQ + y; fsg + row
+// offset + (c K + k) 8 is f.
 template <int K>
-__device__ __forceinline__ void slot_phi_cellrows(const double* __restrict__ gv, const uint32_t* __restrict__ eq23,
-                                                  const double* __restrict__ fsg, const SlotEntries& se, int lane,
-                                                  int c, int part, int b2, int b3, double (&phi)[K][K / 4]) {
-    constexpr int C = LbMma<K>::C, KQ = LbMma<K>::KQ;
-    const int k3o = part * KQ;
-#pragma unroll
-    for (int x = 0; x < K; ++x)
-#pragma unroll
-        for (int y = 0; y < KQ; ++y) phi[x][y] = 0.0;
-    const int cb = se.cb, ce = se.ce;
-    if (cb >= ce) return;
+__device__ __forceinline__ void phi_runs(const unsigned char* rec, int n, const unsigned char* fsg, int c, int part,
+                                         double (&phi)[K][K / 4]) {
+    constexpr int KQ = K / 4;
+    const unsigned char* f2c = fsg + c * K * 8;
+    const unsigned char* f3c = f2c + part * KQ * 8;
+    LbRun<double> r;
+    r.read(rec);
     double h[KQ];
 #pragma unroll
-    for (int y = 0; y < KQ; ++y) h[y] = 0.0;
-    int cur = -1;
-    auto flush = [&]() {
-        const double2* __restrict__ f2p = reinterpret_cast<const double2*>(fsg + ((size_t)cur * C + c) * K);
+    for (int y = 0; y < KQ; ++y)
+        h[y] = fma(r.gb, reinterpret_cast<const double*>(f3c + r.off3b)[y],
+                   r.ga * reinterpret_cast<const double*>(f3c + r.off3a)[y]);
+#pragma unroll 1
+    for (int i = 1; i <= n; ++i) {
+        const double2* f2p = reinterpret_cast<const double2*>(f2c + r.off2);
+        if (i < n) rec += LbRun<double>::BYTES;  // the last pass reads the last run again
+        r.read(rec);
+        double fa[KQ], fb[KQ];
+#pragma unroll
+        for (int y = 0; y < KQ; ++y) {
+            fa[y] = reinterpret_cast<const double*>(f3c + r.off3a)[y];
+            fb[y] = reinterpret_cast<const double*>(f3c + r.off3b)[y];
+        }
 #pragma unroll
         for (int x = 0; x < K / 2; ++x) {
             const double2 f2 = f2p[x];
@@ -953,34 +955,48 @@ __device__ __forceinline__ void slot_phi_cellrows(const double* __restrict__ gv,
             }
         }
 #pragma unroll
-        for (int y = 0; y < KQ; ++y) h[y] = 0.0;
-    };
-    for (int eb = cb; eb < ce; eb += 32) {
-        const int nb = min(32, ce - eb);
-        uint32_t my_q23 = se.q23;
-        double my_g = se.g;
-        if (eb != cb) {
-            my_q23 = 0;
-            my_g = 0.0;
-            if (lane < nb) {
-                my_q23 = __ldg(eq23 + eb + lane);
-                my_g = __ldg(gv + eb + lane);
-            }
-        }
-        for (int j = 0; j < nb; ++j) {
-            const uint32_t q23 = __shfl_sync(0xffffffffu, my_q23, j);
-            const double g = __shfl_sync(0xffffffffu, my_g, j);
-            const int q2 = (int)(q23 & 0xffffu) - b2, q3 = (int)(q23 >> 16) - b3;
-            if (q2 != cur) {
-                if (cur >= 0) flush();
-                cur = q2;
-            }
-            const double* __restrict__ f3p = fsg + ((size_t)q3 * C + c) * K + k3o;
-#pragma unroll
-            for (int y = 0; y < KQ; ++y) h[y] = fma(g, f3p[y], h[y]);
-        }
+        for (int y = 0; y < KQ; ++y) h[y] = fma(r.gb, fb[y], r.ga * fa[y]);
     }
-    if (cur >= 0) flush();
+}
+
+// The same in FP32: lane (cell c, part p) holds the pairs phi[k2 / 2][y], k3 = p + 2 y; fsg + row offset
+// + ((k / 2) C + c) 8 + (k % 2) 4 is f.
+template <int K>
+__device__ __forceinline__ void phi_runs(const unsigned char* rec, int n, const unsigned char* fsg, int c, int part,
+                                         unsigned long long (&phi)[K / 2][K / 2]) {
+    constexpr int KQ = K / 2, KS = LbShape<K>::C * 8;  // bytes from one k pair to the next
+    const unsigned char* f2c = fsg + c * 8;
+    const unsigned char* f3c = f2c + part * 4;
+    LbRun<float> r;
+    r.read(rec);
+    float h[KQ];
+#pragma unroll
+    for (int y = 0; y < KQ; ++y)
+        h[y] = fmaf(r.gb, *reinterpret_cast<const float*>(f3c + r.off3b + y * KS),
+                    r.ga * *reinterpret_cast<const float*>(f3c + r.off3a + y * KS));
+#pragma unroll 1
+    for (int i = 1; i <= n; ++i) {
+        const unsigned char* f2p = f2c + r.off2;
+        if (i < n) rec += LbRun<float>::BYTES;
+        r.read(rec);
+        float fa[KQ], fb[KQ];
+#pragma unroll
+        for (int y = 0; y < KQ; ++y) {
+            fa[y] = *reinterpret_cast<const float*>(f3c + r.off3a + y * KS);
+            fb[y] = *reinterpret_cast<const float*>(f3c + r.off3b + y * KS);
+        }
+        unsigned long long f2[K / 2];
+#pragma unroll
+        for (int x = 0; x < K / 2; ++x) f2[x] = *reinterpret_cast<const unsigned long long*>(f2p + x * KS);
+#pragma unroll
+        for (int y = 0; y < KQ; ++y) {
+            const unsigned long long hh = pack2(h[y], h[y]);
+#pragma unroll
+            for (int x = 0; x < K / 2; ++x) ffma2(phi[x][y], f2[x], hh);
+        }
+#pragma unroll
+        for (int y = 0; y < KQ; ++y) h[y] = fmaf(r.gb, fb[y], r.ga * fa[y]);
+    }
 }
 
 __device__ __forceinline__ void lb_dmma(double& d0, double& d1, double a, double b) {
@@ -989,14 +1005,15 @@ __device__ __forceinline__ void lb_dmma(double& d0, double& d1, double a, double
                  : "d"(a), "d"(b));
 }
 
-enum { LBI_TR = 0, LBI_ORD, LBI_BEGIN, LBI_END };  // item: t | row << 16, ord | l2 << 16 | l3 << 24, entries
+enum { LBI_TR = 0, LBI_ORD, LBI_BEGIN, LBI_END };  // item: t | row << 16, ord, its run records
 enum { LBU_L1 = 0, LBU_BROWS, LBU_TLOFF, LBU_NT, LBU_ITOFF, LBU_NIT, LBU_INTS = 8 };
 
-template <int K, int C, typename T, int W, bool MMA = false>
+template <int K, int C, typename T, int W>
 __device__ __forceinline__ void lblock_body(const SplitArgs& a) {
-    using S = LbShape<K, C, T>;
-    static_assert(!MMA || (C == LbMma<K>::C && sizeof(T) == 8), "the FP64 tensor-core K^3 step takes 8 FP64 cells");
-    constexpr int KH = S::KH, KQ = S::KQ, PS = S::PS, RTB = MMA ? LbMma<K>::RT_BYTES : S::RT_BYTES;
+    constexpr bool MMA = sizeof(T) == 8;
+    static_assert(C == (MMA ? LbMma<K>::C : LbShape<K>::C), "8 FP64 or 16 FP32 cells");
+    constexpr int RTB = MMA ? LbMma<K>::RT_BYTES : LbShape<K>::RT_BYTES;
+    constexpr int RB = LbRun<T>::BYTES;
     constexpr int ROWB = K * C * (int)sizeof(T);
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* ring = smem + a.off_b;
@@ -1026,6 +1043,16 @@ __device__ __forceinline__ void lblock_body(const SplitArgs& a) {
     const T* __restrict__ pcg = reinterpret_cast<const T*>(a.pf) + (size_t)cg * M * C;
     const T* __restrict__ rsrc = reinterpret_cast<const T*>(a.rfp64);
     const int4* __restrict__ items = a.items + it_off;
+    unsigned char* wrec = smem + a.off_rec + (tid >> 5) * 2 * kLbRecs * RB;  // the warp's record buffers
+
+    // the records [rb, min(re, rb + kLbRecs)) into buffer `buf`, as one copy group
+    auto fetch_recs = [&](int rb, int re, int buf) {
+        const int n16 = min(re - rb, kLbRecs) * (RB / 16);
+        if (lane < n16)
+            cp_async16(wrec + buf * kLbRecs * RB + lane * 16, a.recs + (size_t)rb * (RB / 16) + lane);
+        cp_async_commit();
+    };
+    static_assert(kLbRecs * RB / 16 <= 32, "a lane per 16 bytes");
 
     auto issue = [&](int ti, int sb) {
         const int t = a.band_tl[tl_off + ti];
@@ -1069,17 +1096,13 @@ __device__ __forceinline__ void lblock_body(const SplitArgs& a) {
     };
     int cur_i = grab();
     int4 it = cur_i < n_it ? __ldg(items + cur_i) : make_int4(0, 0, 0, 0);
-    SlotEntries se = cur_i < n_it ? slot_fetch(a, a.e_g, it.z, it.w, lane) : SlotEntries{0, 0, 0u, 0.0};
+    int buf = 0;
+    fetch_recs(it.z, it.w, buf);
     while (cur_i < n_it) {
         const int nxt_i = grab();
         int4 nit = make_int4(0, 0, 0, 0);
-        SlotEntries nse{0, 0, 0u, 0.0};
-        if (nxt_i < n_it) {
-            nit = __ldg(items + nxt_i);
-            nse = slot_fetch(a, a.e_g, nit.z, nit.w, lane);
-        }
-        const int ti = it.x & 0xffff, row = it.x >> 16, ord = it.y & 0xffff;
-        const int l2 = (it.y >> 16) & 0xff, l3 = (it.y >> 24) & 0xff;
+        if (nxt_i < n_it) nit = __ldg(items + nxt_i);
+        const int ti = it.x & 0xffff, row = it.x >> 16, ord = it.y;
         const int sb = ti % D;
         if (lane == 0) {
             const long long t0 = clock64();
@@ -1096,14 +1119,28 @@ __device__ __forceinline__ void lblock_body(const SplitArgs& a) {
         bool ok = wait_bar(&bfull[sb], (uint32_t)((ti / D) & 1), abort_flag, a.err, a.wait_cycles);
         if (ok) {
             const unsigned char* st = ring + (size_t)sb * a.stage_bytes;
-            const int b2 = l2 * l2, b3 = l3 * l3 - (l3 != l2 ? 2 * l2 + 1 : 0);
-            T acc[K];
+            // the item's runs, a buffer at a time; the buffer after the last holds the next item's first runs
+            auto run_all = [&](auto& phi) {
+                for (int rb = it.z; rb < it.w; rb += kLbRecs) {
+                    const bool more = rb + kLbRecs < it.w;
+                    fetch_recs(more ? rb + kLbRecs : nit.z, more ? it.w : nit.w, buf ^ 1);
+                    cp_async_wait<1>();
+                    __syncwarp();
+                    phi_runs<K>(wrec + buf * kLbRecs * RB, min(it.w - rb, kLbRecs), st + RTB, c, part, phi);
+                    __syncwarp();
+                    buf ^= 1;
+                }
+            };
+            float acc[MMA ? 1 : K / 2];
             double dq[MMA ? LbMma<K>::MT : 1][2];
             if constexpr (MMA) {
                 constexpr int MT = LbMma<K>::MT, SS = LbMma<K>::S, QQ = LbMma<K>::KQ;
                 double phi[K][QQ];
-                slot_phi_cellrows<K>(a.e_g, a.e_q23, reinterpret_cast<const double*>(st + RTB), se, lane, c, part,
-                                     b2, b3, phi);
+#pragma unroll
+                for (int x = 0; x < K; ++x)
+#pragma unroll
+                    for (int y = 0; y < QQ; ++y) phi[x][y] = 0.0;
+                run_all(phi);
                 const double* __restrict__ ra = reinterpret_cast<const double*>(st) + lane;
                 // two accumulator sets per m-tile (even and odd k-steps): two MMA chains instead of one
                 double d[MT][2][2];
@@ -1122,44 +1159,52 @@ __device__ __forceinline__ void lblock_body(const SplitArgs& a) {
                     dq[mt][1] = d[mt][0][1] + d[mt][1][1];
                 }
             } else {
-                T phi[KH][KQ];
-                slot_phi_staged<K, C, T>(a.e_g, a.e_q23, reinterpret_cast<const T*>(st + RTB), se, lane, c, part, b2,
-                                         b3, phi);
-                const T* rp = reinterpret_cast<const T*>(st) + part * PS;
+                using S = LbShape<K>;
+                unsigned long long phi[K / 2][S::KQ], sum[K / 2];
 #pragma unroll
-                for (int k1 = 0; k1 < K; ++k1) acc[k1] = (T)0;
+                for (int x = 0; x < K / 2; ++x)
 #pragma unroll
-                for (int x = 0; x < KH; ++x)
+                    for (int y = 0; y < S::KQ; ++y) phi[x][y] = 0ull;
+                run_all(phi);
+                const float* rp = reinterpret_cast<const float*>(st) + part * S::PS;
 #pragma unroll
-                    for (int y = 0; y < KQ; ++y) {
-                        const T* rr = rp + (x * KQ + y) * K;
-                        if constexpr (sizeof(T) == 8) {
+                for (int j = 0; j < K / 2; ++j) sum[j] = 0ull;
 #pragma unroll
-                            for (int j = 0; j < K / 2; ++j) {
-                                const double2 r = reinterpret_cast<const double2*>(rr)[j];
-                                acc[2 * j] = fma((T)r.x, phi[x][y], acc[2 * j]);
-                                acc[2 * j + 1] = fma((T)r.y, phi[x][y], acc[2 * j + 1]);
-                            }
-                        } else {
+                for (int x = 0; x < K; ++x)
 #pragma unroll
-                            for (int j = 0; j < K / 4; ++j) {
-                                const float4 r = reinterpret_cast<const float4*>(rr)[j];
-                                acc[4 * j] = fma((T)r.x, phi[x][y], acc[4 * j]);
-                                acc[4 * j + 1] = fma((T)r.y, phi[x][y], acc[4 * j + 1]);
-                                acc[4 * j + 2] = fma((T)r.z, phi[x][y], acc[4 * j + 2]);
-                                acc[4 * j + 3] = fma((T)r.w, phi[x][y], acc[4 * j + 3]);
-                            }
+                    for (int y = 0; y < S::KQ; ++y) {
+                        const float2 v = unpack2(phi[x / 2][y]);
+                        const unsigned long long vv = x % 2 ? pack2(v.y, v.y) : pack2(v.x, v.x);
+                        const ulonglong2* rr = reinterpret_cast<const ulonglong2*>(rp + (x * S::KQ + y) * K);
+#pragma unroll
+                        for (int j = 0; j < K / 4; ++j) {
+                            const ulonglong2 r = rr[j];
+                            ffma2(sum[2 * j], r.x, vv);
+                            ffma2(sum[2 * j + 1], r.y, vv);
                         }
                     }
-            }
-            // the parts of a cell sit in lanes c, c + C, c + 2C, ...: sum them, then part p adds the
-            // k1 of its quarter once this row's earlier slices are in (the MMA has summed them already)
-            if constexpr (!MMA) {
+                // the two parts of a cell sit in lanes c and c + C: part p keeps k1 = p K/2 .. and hands
+                // the other half over
+                float first[K / 2], second[K / 2];
 #pragma unroll
-                for (int k1 = 0; k1 < K; ++k1)
+                for (int j = 0; j < K / 2; ++j) {
+                    const float2 v = unpack2(sum[j]);
+                    const int at = 2 * j % (K / 2);
+                    if (2 * j < K / 2) {
+                        first[at] = v.x;
+                        first[at + 1] = v.y;
+                    } else {
+                        second[at] = v.x;
+                        second[at + 1] = v.y;
+                    }
+                }
 #pragma unroll
-                    for (int o = C; o < 32; o <<= 1) acc[k1] += __shfl_xor_sync(0xffffffffu, acc[k1], o);
+                for (int j = 0; j < K / 2; ++j) {
+                    const float got = __shfl_xor_sync(0xffffffffu, part ? first[j] : second[j], C);
+                    acc[j] = (part ? second[j] : first[j]) + got;
+                }
             }
+            // added once this row's earlier slices are in
             if (lane == 0) {
                 const long long t0 = clock64();
                 while (ticket[row] != ord) {
@@ -1187,11 +1232,9 @@ __device__ __forceinline__ void lblock_body(const SplitArgs& a) {
                         }
                     }
                 } else {
-                    double* qr = qacc + (size_t)row * K * C + c;
-                    constexpr int KP = K / (32 / C);  // k1 per part
+                    double* qr = qacc + ((size_t)row * K + part * (K / 2)) * C + c;
 #pragma unroll
-                    for (int k1 = 0; k1 < K; ++k1)
-                        if (k1 / KP == part) qr[k1 * C] += (double)acc[k1];
+                    for (int j = 0; j < K / 2; ++j) qr[j * C] += (double)acc[j];
                 }
             }
             __syncwarp();
@@ -1214,8 +1257,8 @@ __device__ __forceinline__ void lblock_body(const SplitArgs& a) {
         __syncwarp();
         cur_i = nxt_i;
         it = nit;
-        se = nse;
     }
+    cp_async_wait<0>();
     __syncthreads();
     if (*abort_flag) return;
     // Q += the band's rows of the CTA's cells (cell-major, in place)
@@ -1230,7 +1273,7 @@ __device__ __forceinline__ void lblock_body(const SplitArgs& a) {
 // added into the FP64 Q rows): 16 cells per CTA, the same shared memory.
 template <int K>
 __global__ void __launch_bounds__(kLbWarps * 32, 1) af_lblock64_kernel(SplitArgs a) {
-    lblock_body<K, kLbCells, double, kLbWarps, true>(a);
+    lblock_body<K, kLbCells, double, kLbWarps>(a);
 }
 template <int K>
 __global__ void __launch_bounds__(kLbWarps * 32, 1) af_lblock32_kernel(SplitArgs a) {
@@ -1534,12 +1577,14 @@ struct SplitPlan {
     int lb_bands = 0, lb_rows = 0, lb_t = 0;  // bands, rows of the largest band, longest t-list
     int lb_ring = 0, lb_stage = 0;    // stages in the ring, bytes per stage (FP64, 8 cells per CTA)
     int lb32_ring = 0, lb32_stage = 0;  // the same for the FP32 forms (16 cells per CTA)
-    float* d_rfl32 = nullptr;         // FP32 R_t as [part][e][k1] for 16 cells per CTA
+    float* d_rfl32 = nullptr;         // the FP32 l-block kernel: R_t as LbShape::r_at
     Layout laylb32{};
     int* d_lb_units = nullptr;        // per band: LBU_INTS ints
     int* d_lb_order = nullptr;        // bands, heaviest first
     int4* d_lb_items = nullptr;       // per band: its (t, row) slices in t-major order
     int* d_lb_titems = nullptr;       // per t-list position: its items
+    uint4* d_lb_recs = nullptr;       // run records of the items, FP64 and FP32 (LbRun)
+    uint4* d_lb_recs32 = nullptr;
     Layout lay{};
     Layout lay64{};
     Layout laybf{};
@@ -1697,20 +1742,16 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
     std::vector<double> rfl;
     std::vector<float> rfl32;
     if constexpr (lblock_supported_k(K)) {
-        auto fill = [&](auto shape, auto& out) {
-            using S8 = decltype(shape);
-            out.assign((size_t)NL * S8::P * S8::PS, 0);
-            for (int t = 0; t < NL; ++t)
-                for (int pp = 0; pp < S8::P; ++pp)
-                    for (int e = 0; e < S8::E; ++e) {
-                        const int k2 = e / S8::KQ, k3 = S8::k3(pp, e % S8::KQ);
+        using S32 = LbShape<K>;
+        rfl32.assign((size_t)NL * S32::P * S32::PS, 0.0f);
+        for (int t = 0; t < NL; ++t)
+            for (int pp = 0; pp < S32::P; ++pp)
+                for (int y = 0; y < S32::KQ; ++y)
+                    for (int k2 = 0; k2 < K; ++k2)
                         for (int k1 = 0; k1 < K; ++k1)
-                            out[((size_t)t * S8::P + pp) * S8::PS + (size_t)e * K + k1] =
-                                (typename std::decay_t<decltype(out)>::value_type)R[(size_t)t * K * K * K + k1 +
-                                                                                   (size_t)K * k2 + (size_t)K * K * k3];
-                    }
-        };
-        fill(LbShape<K, 2 * kLbCells, float>{}, rfl32);
+                            rfl32[(size_t)t * S32::P * S32::PS + S32::r_at(pp, k1, k2, y)] =
+                                (float)R[(size_t)t * K * K * K + k1 + (size_t)K * k2 +
+                                         (size_t)K * K * (pp + y * S32::P)];
         // FP64: A fragments of the m8n8k4 MMAs, [t][m-tile][k-step][lane] (LbMma)
         using LM = LbMma<K>;
         rfl.assign((size_t)NL * LM::MT * LM::S * 32, 0.0);
@@ -1817,7 +1858,20 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
     // its row's slices (the row's ticket) and the (l2, l3) of its t
     std::vector<int> units_lb, order_lb, titems_lb(band_tl.size(), 0);
     std::vector<int4> items_lb;
+    std::vector<uint4> recs64, recs32;  // run records (LbRun), two words of 16 bytes per run in FP64
     std::vector<double> work_lb;
+    constexpr uint32_t kRowB = K * kLbCells * sizeof(double);  // = K 16 sizeof(float)
+    auto add_run = [&](double ga, double gb, uint32_t r2, uint32_t r3a, uint32_t r3b) {
+        uint32_t g[4];
+        std::memcpy(g, &ga, 8);
+        std::memcpy(g + 2, &gb, 8);
+        recs64.push_back(make_uint4(g[0], g[1], g[2], g[3]));
+        recs64.push_back(make_uint4(r2 * kRowB, r3a * kRowB, r3b * kRowB, 0u));
+        const float fa = (float)ga, fb = (float)gb;
+        std::memcpy(g, &fa, 4);
+        std::memcpy(g + 1, &fb, 4);
+        recs32.push_back(make_uint4(g[0], g[1], r2 * kRowB, (r3a * kRowB / 16) | (r3b * kRowB / 16) << 16));
+    };
     int lb_rows = 0, lb_t = 0;
     bool lb_ok = L < 128;
     for (const BandInfo& bd : bands) {
@@ -1825,12 +1879,22 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
         std::vector<int> ord(bd.brows, 0);
         for (int ti = 0; ti < bd.n_t; ++ti) {
             const int t = band_tl[bd.tl_off + ti];
-            const int l23 = t_l23[t];
+            const int l2 = t_l23[t] & 0xff, l3 = t_l23[t] >> 8;
+            // first q of the stage's rows: band l2, then (unless it is the same) band l3
+            const uint32_t b2 = l2 * l2, b3 = l3 * l3 - (l3 != l2 ? 2 * l2 + 1 : 0);
             for (int r = 0; r < bd.brows; ++r) {
                 const int sl = band_slice[bd.tab_off + (size_t)ti * bd.brows + r];
                 if (sl < 0) continue;
-                items_lb.push_back(make_int4(ti | (r << 16), ord[r]++ | ((l23 & 0xff) << 16) | ((l23 >> 8) << 24),
-                                              slice_e[sl], slice_e[sl + 1]));
+                const int run0 = (int)(recs32.size());
+                if (lblock_supported_k(K))
+                    for (int z = slice_e[sl]; z < slice_e[sl + 1];) {
+                        const uint32_t q2 = e_q23[z] & 0xffffu, q3 = e_q23[z] >> 16;
+                        const bool two = z + 1 < slice_e[sl + 1] && (e_q23[z + 1] & 0xffffu) == q2;
+                        add_run(e_g[z], two ? e_g[z + 1] : 0.0, q2 - b2, q3 - b3,
+                                (two ? e_q23[z + 1] >> 16 : q3) - b3);
+                        z += two ? 2 : 1;
+                    }
+                items_lb.push_back(make_int4(ti | (r << 16), ord[r]++, run0, (int)recs32.size()));
                 ++titems_lb[bd.tl_off + ti];
             }
         }
@@ -1889,20 +1953,19 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
         // FP64, 8 cells; FP32, 16 cells: the same bytes per f row
         const int stage = (LbMma<K>::RT_BYTES + max_rows * K * kLbCells * (int)sizeof(double) + 127) / 128 * 128;
         const int stage32 =
-            (LbShape<K, 2 * kLbCells, float>::RT_BYTES + max_rows * K * 2 * kLbCells * (int)sizeof(float) + 127) / 128 *
-            128;
+            (LbShape<K>::RT_BYTES + max_rows * K * 2 * kLbCells * (int)sizeof(float) + 127) / 128 * 128;
         int ring = kLbMaxRing, ring32 = kLbMaxRing;
-        while (ring >= 2 && lblock_layout(ring, stage, K, lb_rows, lb_t, kLbCells).total > optin) --ring;
-        while (ring32 >= 2 && lblock_layout(ring32, stage32, K, lb_rows, lb_t, 2 * kLbCells).total > optin) --ring32;
+        while (ring >= 2 && lblock_layout(ring, stage, K, lb_rows, lb_t, kLbCells, LbRun<double>::BYTES).total > optin) --ring;
+        while (ring32 >= 2 && lblock_layout(ring32, stage32, K, lb_rows, lb_t, 2 * kLbCells, LbRun<float>::BYTES).total > optin) --ring32;
         if (ring >= 2) {
             sp->lb_ring = ring;
             sp->lb_stage = stage;
-            sp->laylb = lblock_layout(ring, stage, K, lb_rows, lb_t, kLbCells);
+            sp->laylb = lblock_layout(ring, stage, K, lb_rows, lb_t, kLbCells, LbRun<double>::BYTES);
         }
         if (ring32 >= 2) {
             sp->lb32_ring = ring32;
             sp->lb32_stage = stage32;
-            sp->laylb32 = lblock_layout(ring32, stage32, K, lb_rows, lb_t, 2 * kLbCells);
+            sp->laylb32 = lblock_layout(ring32, stage32, K, lb_rows, lb_t, 2 * kLbCells, LbRun<float>::BYTES);
         }
     }
     sp->laybf = bf16_layout<K, C>(NQ);
@@ -1930,6 +1993,8 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
         (ce = upload_vec(&sp->d_lb_order, order_lb, bytes)) != cudaSuccess ||
         (ce = upload_vec(&sp->d_lb_items, items_lb, bytes)) != cudaSuccess ||
         (ce = upload_vec(&sp->d_lb_titems, titems_lb, bytes)) != cudaSuccess ||
+        (ce = upload_vec(&sp->d_lb_recs, recs64, bytes)) != cudaSuccess ||
+        (ce = upload_vec(&sp->d_lb_recs32, recs32, bytes)) != cudaSuccess ||
         (ce = upload_vec(&sp->d_t_l23, t_l23, bytes)) != cudaSuccess)
         return fail_split(ce == cudaErrorMemoryAllocation ? CF_ENOMEM : CF_ECUDA,
                           std::string("split form: upload: ") + cudaGetErrorString(ce));
@@ -2031,7 +2096,7 @@ int run64_impl(const SplitPlan* sp, double* q_cm, const double* f_cm, int64_t B,
     return CF_OK;
 }
 
-// Bytes of the packed f that the l-block kernels read: [ceil(B / C)][N_Q][K][C] of T.
+// Bytes of the packed f that the l-block kernels read: [ceil(B / C)][N_Q] rows of K C values of T.
 size_t lblock_pack_bytes_of(int n_q, int k, int64_t B, bool f32) {
     const int C = f32 ? 2 * kLbCells : kLbCells;
     return (size_t)((B + C - 1) / C) * (size_t)n_q * k * C * (f32 ? sizeof(float) : sizeof(double));
@@ -2075,6 +2140,7 @@ int runlb_impl(const SplitPlan* sp, double* q_cm, const double* f_cm, void* pf, 
     a.band_tl = sp->d_band_tl;
     a.items = sp->d_lb_items;
     a.t_items = sp->d_lb_titems;
+    a.recs = F32 ? sp->d_lb_recs32 : sp->d_lb_recs;
     a.pf = static_cast<const double*>(pf);  // read as T by the kernel
     a.t_l23 = sp->d_t_l23;
     a.q = q_cm;
@@ -2093,6 +2159,7 @@ int runlb_impl(const SplitPlan* sp, double* q_cm, const double* f_cm, void* pf, 
     a.off_red = lay.off_red;
     a.off_bar = lay.off_bar;
     a.off_misc = lay.off_misc;
+    a.off_rec = lay.off_rec;
     const long long blocks = (long long)sp->lb_bands * n_cg;
     kern<<<(unsigned)blocks, W * 32, lay.total, st>>>(a);
     e = cudaGetLastError();
@@ -2258,7 +2325,7 @@ void split_destroy(SplitPlan* sp) {
     void* ptrs[] = {sp->d_rplanes, sp->d_e_gs, sp->d_rb_off, sp->d_rb_gs, sp->d_rb_l23, sp->d_units, sp->d_unit_order, sp->d_band_tl,
                     sp->d_band_rng, sp->d_err, sp->d_rfp64, sp->d_rbf, sp->d_units64, sp->d_unit_order64,
                     sp->d_rbf8, sp->d_rfl, sp->d_rfl32, sp->d_t_l23, sp->d_lb_units, sp->d_lb_order, sp->d_lb_items,
-                    sp->d_lb_titems};
+                    sp->d_lb_titems, sp->d_lb_recs, sp->d_lb_recs32};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete sp;

@@ -36,6 +36,7 @@ struct DevOp {
     // outer-product kernels (K <= 8): per slice (t, first chunk, chunks with a second q3, chunks); per chunk
     // 4 x (q2, q3a, q3b) and 4 x G of both; R_t in lane order (null where the plan has no such tables)
     const int* x_q1;  // [N_Q + 1] x_slice range of each q1
+    const int* x_cum;  // [n_items + 1] work of the rows item_q1[0 .. i) added up
     const int4* x_slice;
     const unsigned char* x_chunk;
     const double2* x_R;

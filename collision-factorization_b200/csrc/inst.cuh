@@ -194,7 +194,7 @@ static LaunchResult launch_outer(const LaunchArgs& a) {
     const OuterFit fit = outer_fit(a.op.n_q, K, JV, a.max_smem);
     const int path = fit.nc == 16 ? PATH_TILE : PATH_TILE4;
     const bool stream = a.ss && a.ss->ready;
-    if (a.op.x_slice == nullptr || a.counter == nullptr || fit.nc == 0 || (stream && fit.nc != 16))
+    if (a.op.x_slice == nullptr || a.op.n_items == 0 || a.counter == nullptr || fit.nc == 0 || (stream && fit.nc != 16))
         return {-1, 0, cudaSuccess, path};
     OuterGeom g;
     g.nc = fit.nc;
@@ -208,13 +208,16 @@ static LaunchResult launch_outer(const LaunchArgs& a) {
     const int64_t ctas = (int64_t)per_sm * a.n_sms;
     const int64_t n_ht = (a.n_cells + g.nc - 1) / g.nc;
     if (n_ht > INT32_MAX / 16) return {2, 0, cudaSuccess, path};
-    // streamed: every half-tile in 4, so that the first chunk gives work to every CTA; sixteenths at the end from
-    // 4 rows each on (L = 10, K = 8, 300 cells: J.v 393 against 610 us; 4096 cells: Q 1542 against 1555 us)
-    const UnitCuts cuts = stream ? UnitCuts{0, (int)n_ht, (int)n_ht * 4} : cut_units(n_ht, ctas, a.op.n_items >= 64);
+    // streamed: every half-tile in 4, so that the first chunk gives work to every CTA
+    const UnitCuts cuts{0, (int)n_ht, (int)n_ht * 4};
     const OuterSched sc{a.bin_begin, a.bin_q1, cuts, a.counter};
-    e = cudaMemsetAsync(a.counter, 0, sizeof(int), a.stream);
-    if (e != cudaSuccess) return {5, 0, e, path};
-    const unsigned grid = (unsigned)std::min<int64_t>(cuts.n_units, ctas);
+    if (stream) {
+        e = cudaMemsetAsync(a.counter, 0, sizeof(int), a.stream);
+        if (e != cudaSuccess) return {5, 0, e, path};
+    }
+    // few units: whole numbers of CTAs for each (L = 7, K = 8, 64 cells: J.v 47 against 68 us)
+    const int64_t most = !stream && ctas >= 8 * n_ht ? ctas / n_ht * n_ht : ctas;
+    const unsigned grid = (unsigned)std::min<int64_t>(stream ? cuts.n_units : n_ht * a.op.n_items, most);
     const StreamSync none{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, 0};
     kern<<<grid, kOuterWarps * 32, smem, a.stream>>>(a.op, sc, g, a.ss ? *a.ss : none, g.tiled ? a.fT : a.f_cm,
                                                     g.tiled ? a.vT : a.v_cm, g.tiled ? a.QT : a.q_cm,
@@ -494,7 +497,7 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
     if (a.ss) {
         if (a.what == OP_RF || a.exact || a.f32) return {8, 0, cudaSuccess, PATH_TILE};
         if constexpr (outer_for(K)) {
-            if (a.path == PATH_AUTO && outer_takes(a.op.n_q, K, a.tile_first, a.n_cells, a.n_sms)) {
+            if (a.path == PATH_AUTO && outer_takes(a.op.n_q, K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms)) {
                 const LaunchResult r = a.what == OP_JV ? launch_outer<K, true>(a) : launch_outer<K, false>(a);
                 if (r.status != -1) return r;
             }
@@ -557,7 +560,7 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
         return launch_for_k<K>(b);
     }
     if constexpr (outer_for(K)) {
-        if (a.path == PATH_AUTO && !a.exact && outer_takes(a.op.n_q, K, a.tile_first, a.n_cells, a.n_sms)) {
+        if (a.path == PATH_AUTO && !a.exact && outer_takes(a.op.n_q, K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms)) {
             const LaunchResult r = jv ? launch_outer<K, true>(a) : launch_outer<K, false>(a);
             if (r.status != -1) return r;
         }

@@ -100,12 +100,12 @@ constexpr bool pair_fits(int n_q, int K, bool jv, size_t max_smem) {
 // K that the outer-product kernels (outer_kernels.cuh) take.
 constexpr bool outer_for(int K) { return K >= 7 && K <= 8; }
 
-// Where they are the faster family (B200, us, outer / tile or pair): from L = 7 on, at every batch (folded Q, K = 8: L = 10,
-// 4096 cells 1542 / 1642, L = 13, 1000 cells 1122 / 1928; J.v, L = 10: 2193 / 3060); below, for batches of at most half
-// an SM's half-tile each (L = 5, 300 cells: 45 / 59; 4096 cells: 205 / 191), whose rows their teams spread better;
-// and the plain K = 8 forms always (L = 5, 4096 cells: 305 / 335).
-constexpr bool outer_takes(int n_q, int K, bool folded, int64_t n_cells, int n_sms) {
-    return outer_for(K) && (n_q >= 64 || (K == 8 && !folded) || (n_cells + 15) / 16 * 2 <= n_sms);
+// Where they are the faster family (B200, us, outer / tile or pair): nearly everywhere (folded Q, K = 8: L = 10, 4096
+// cells 1509 / 1642, L = 13, 1000 cells 1045 / 1928, L = 6, 2048 cells 161 / 176, L = 3, 2000 cells 39 / 51; J.v, L = 10,
+// 2174 / 3060; plain Q, K = 7, L = 5, 4096 cells 250 / 266).  The pair kernel keeps the plain J.v at K = 7 below L = 7
+// (L = 4, 4000 cells: 189 / 176; L = 6, 2000 cells: 312 / 299) unless the batch has at most half a half-tile per SM.
+constexpr bool outer_takes(int n_q, int K, bool folded, bool jv, int64_t n_cells, int n_sms) {
+    return outer_for(K) && (K == 8 || folded || !jv || n_q >= 64 || (n_cells + 15) / 16 * 2 <= n_sms);
 }
 
 // Shared-memory geometry of the outer-product kernels.  Cells lie in pairs, [pair][k][q][cell of the pair],

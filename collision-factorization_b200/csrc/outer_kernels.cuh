@@ -21,8 +21,8 @@
 // What bounds it: shared-memory wavefronts (72 % of peak at L = 10, K = 8: 17 a cell and slice for the Phi operands,
 // 8 for R_t, 8 for chunks, heads and copies), with the FP64 pipe at 50 %.  Four cells a warp (128 registers,
 // 16 warps) rather than eight (255, 8 warps, half the R_t wavefronts): 1591 against 1847 us, latency; R_t read
-// from L2 by each warp instead of staged: 2184 us.  B200, folded, L = 10, K = 8, 4096 cells: Q 1542 us (tile kernel
-// 1642), J.v 2193 us (quarter-tile kernel 3060); L = 13, 1000 cells: Q 1122 us (1928); L = 10, 300 cells: 193 us (285).
+// from L2 by each warp instead of staged: 2184 us.  B200, folded, L = 10, K = 8, 4096 cells: Q 1509 us (tile kernel
+// 1642), J.v 2174 us (quarter-tile kernel 3060); L = 13, 1000 cells: Q 1045 us (1928); L = 10, 300 cells: 158 us (285).
 #pragma once
 #include <type_traits>
 
@@ -31,11 +31,16 @@
 
 namespace cf {
 
+// Work of one launch.  The units' rows, heaviest first, unit after unit, are one list that the CTAs share out in
+// contiguous stretches of equal work (x_cum): at most two cut units a CTA, so teams run out of rows twice and f is
+// staged little more than once.  Against whole units, then quarters, then sixteenths from a counter (B200, us):
+// folded K = 8: L = 10, 4096 cells 1542 -> 1509, 300 cells 193 -> 158; L = 8, 2048 cells: J.v 543 -> 502; L = 13, 1000
+// cells: 1120 -> 1045.  A streamed launch keeps quarters in order of arrival, so that every chunk gives work to all CTAs.
 struct OuterSched {
-    const int* bin_begin;  // as TileSched
+    const int* bin_begin;  // as TileSched (streamed)
     const int* bin_q1;
-    UnitCuts cuts;
-    int* counter;
+    UnitCuts cuts;         // streamed; else n_four units in all
+    int* counter;          // streamed
 };
 
 // Cell layout of one launch.
@@ -283,13 +288,41 @@ __global__ void __launch_bounds__(kOuterWarps * 32, 1)
     OuterTask* tasks = reinterpret_cast<OuterTask*>(rings + 2 * (W / team_warps));
     const size_t mine = (size_t)w_in_team * (kOuterCells / 2) * outer_pair(K, NQP);  // this warp's cells
     int staged = -1;
-    for (;;) {
-        if (tid == 0) s_unit = atomicAdd(sc.counter, 1);
+    // not streamed: what is left of this CTA's stretch, from row s_from.y of unit s_from.x to row s_to.y of unit s_to.x
+    __shared__ int2 s_from, s_to;
+    if (!ss.ready) {
+        const int n = op.n_items;  // <= N_Q <= 268 < the CTA's threads
+        const long long total = op.x_cum[n], work = total * sc.cuts.n_four;
+        // the row boundary nearest to a place in the list
+        auto cut = [&](int i) {
+            const long long at = work * i / gridDim.x;
+            const int u = (int)(at / total), rem = (int)(at - u * total);
+            const int r = __syncthreads_count(tid < n && op.x_cum[tid] + op.x_cum[min(tid, n - 1) + 1] <= 2 * rem);
+            return r == n ? make_int2(u + 1, 0) : make_int2(u, r);
+        };
+        const int2 from = cut(blockIdx.x), to = cut(blockIdx.x + 1);
+        if (tid == 0) {
+            s_from = from;
+            s_to = to;
+        }
         __syncthreads();
-        const int u = s_unit;
-        if (u >= sc.cuts.n_units) break;
-        int ht, bin;
-        unit_of(sc.cuts, u, ht, bin);
+    }
+    for (;;) {
+        int ht, b0, nb;
+        if (ss.ready) {
+            if (tid == 0) s_unit = atomicAdd(sc.counter, 1);
+            __syncthreads();
+            if (s_unit >= sc.cuts.n_units) break;
+            int bin;
+            unit_of(sc.cuts, s_unit, ht, bin);
+            b0 = sc.bin_begin[bin];
+            nb = sc.bin_begin[bin + 1] - b0;
+        } else {
+            ht = s_from.x;
+            b0 = s_from.y;
+            if (ht > s_to.x || (ht == s_to.x && b0 >= s_to.y)) break;
+            nb = (ht == s_to.x ? s_to.y : op.n_items) - b0;
+        }
         const int chunk = ss.ready ? ht / ss.ht_per_chunk : 0;
         const long long cell0 = (long long)ht * g.nc;
         if (ht != staged) {
@@ -314,7 +347,6 @@ __global__ void __launch_bounds__(kOuterWarps * 32, 1)
             cp_async_wait_all();
             staged = ht;
         }
-        const int b0 = sc.bin_begin[bin], nb = sc.bin_begin[bin + 1] - b0;
         if (tid == 0) s_next = 0;
         for (int i = tid; i < nb; i += W * 32) {
             OuterTask t;
@@ -339,6 +371,10 @@ __global__ void __launch_bounds__(kOuterWarps * 32, 1)
             });
         if (ss.done) __threadfence();
         __syncthreads();
+        if (!ss.ready) {
+            if (tid == 0) s_from = make_int2(ht + 1, 0);
+            __syncthreads();
+        }
         if (tid == 0 && ss.done) {
             const int h0 = chunk * ss.ht_per_chunk;
             const int c_ht = min(ss.ht_per_chunk, sc.cuts.n_four - h0);

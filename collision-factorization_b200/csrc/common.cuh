@@ -36,11 +36,11 @@ struct DevOp {
     // outer-product kernels (K <= 8): per slice (t, first chunk, chunks with a second q3, chunks); per chunk
     // 4 x (q2, q3a, q3b) and 4 x G of both; R_t in lane order (null where the plan has no such tables)
     const int* x_q1;  // [N_Q + 1] x_slice range of each q1
-    const int* x_cum;  // [n_items + 1] work of the rows item_q1[0 .. i) added up
     const int4* x_slice;
     const unsigned char* x_chunk;
     const double2* x_R;
     const int* item_q1;
+    const long long* item_cum;  // [n_items + 1] work of the rows item_q1[0 .. i) added up (entries; a slice counts K)
     int grouped;  // each slice's entries sorted by q2 (the folded operator); bit 0: the fast Q tile
                   // routine sums G f(q3) over each run of equal q2 before one outer product with
                   // f(q2), bit 1: the fast J.v tile routine does the same with f and v

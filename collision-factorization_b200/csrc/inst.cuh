@@ -68,43 +68,51 @@ static LaunchResult launch_af(const LaunchArgs& a) {
     return {e == cudaSuccess ? 0 : 5, 1, e, PATH_GATHER};
 }
 
+// CTAs of a launch whose rows are shared out in stretches (stretch_cut).  Few units: whole numbers of CTAs for each
+// (L = 7, K = 8, 64 cells: J.v 47 against 68 us), as a stretch of little more than a row should not take one row
+// from each of two units.
+static inline unsigned stretch_grid(const LaunchArgs& a, int64_t n_units, int64_t ctas) {
+    return (unsigned)std::min<int64_t>(n_units * a.op.n_items, ctas >= 8 * n_units ? ctas / n_units * n_units : ctas);
+}
+
 // Tile-resident persistent kernel.  Returns status -1 when it does not fit (shared memory or
 // occupancy), in which case the caller uses the gather kernel.
-template <int K, int W, bool EXACT, bool JV>
+template <int K, int W, bool EXACT, bool JV, bool CM = false>
 static LaunchResult launch_tile(const LaunchArgs& a) {
     const int M = a.op.n_q * K;
-    const size_t smem = tile_smem_bytes<K>(M, W, JV);
-    if (smem + 256 > a.max_smem || a.counter == nullptr) return {-1, 0, cudaSuccess, PATH_TILE};
-    auto kern = af_tile_kernel<K, W, EXACT, JV>;
+    size_t smem = tile_smem_bytes<K>(M, W, JV);
+    if (smem + 256 > a.max_smem || a.op.n_items == 0) return {-1, 0, cudaSuccess, PATH_TILE};
+    auto kern = af_tile_kernel<K, W, EXACT, JV, CM>;
     int per_sm = 0;
     cudaError_t e = resident_ctas((const void*)kern, W * 32, smem, &per_sm);
     if (e != cudaSuccess) return {5, 0, e, PATH_TILE};
     if (per_sm < 1) return {-1, 0, cudaSuccess, PATH_TILE};
-    const int64_t ctas = (int64_t)per_sm * a.n_sms;
     const int64_t n_ht = (a.n_cells + kTileCells - 1) / kTileCells;
-    TileSched sc;
-    sc.bin_begin = a.bin_begin;
-    sc.bin_q1 = a.bin_q1;
-    sc.n_ht = (int)n_ht;
-    const int64_t n_whole = n_ht > ctas ? n_ht - ctas : 0;
-    const int64_t rem = n_ht - n_whole;
-    sc.split = rem * 4 >= ctas ? 4 : 16;
-    sc.n_whole = (int)n_whole;
-    const int64_t n_units = n_whole + rem * sc.split;
-    if (n_units > INT32_MAX) return {2, 0, cudaSuccess, PATH_TILE};
-    sc.n_units = (int)n_units;
-    sc.counter = a.counter;
-    e = cudaMemsetAsync(a.counter, 0, sizeof(int), a.stream);
-    if (e != cudaSuccess) return {5, 0, e, PATH_TILE};
-    const unsigned grid = (unsigned)(n_units < ctas ? n_units : ctas);
-    kern<<<grid, W * 32, smem, a.stream>>>(a.op, sc, a.fT, a.vT, a.QT);
+    if (n_ht > INT32_MAX / 16) return {2, 0, cudaSuccess, PATH_TILE};
+    const unsigned grid = stretch_grid(a, n_ht, (int64_t)per_sm * a.n_sms);
+    // as many half-tiles of a stretch at a time as fit beside each other, without an SM losing a CTA
+    int n_buf = (int)std::min<int64_t>(kTileBufs, (n_ht + grid - 1) / grid + 1);
+    while (n_buf > 1) {
+        int with = 0;
+        const size_t more = tile_smem_bytes<K>(M, W, JV, n_buf);
+        if (more + 256 <= a.max_smem) {
+            e = resident_ctas((const void*)kern, W * 32, more, &with);
+            if (e != cudaSuccess) return {5, 0, e, PATH_TILE};
+        }
+        if (with >= per_sm) {
+            smem = more;
+            break;
+        }
+        --n_buf;
+    }
+    kern<<<grid, W * 32, smem, a.stream>>>(a.op, (int)n_ht, n_buf, CM ? a.f_cm : a.fT, CM ? a.v_cm : a.vT,
+                                           CM ? a.q_cm : a.QT, (long long)a.n_cells);
     e = cudaGetLastError();
     return {e == cudaSuccess ? 0 : 5, 1, e, PATH_TILE};
 }
 
-// Tile kernel on cell-major f and Q (a.f_cm, a.q_cm).  Streamed (a.ss->ready set): every half-tile
-// split into 4 q1 bins, chunk flags in a.ss.  Resident (a.ss->ready null): the tile kernel's own
-// schedule, no waits.  Status -1 when the tile does not fit.
+// Tile kernel on cell-major f and Q (a.f_cm, a.q_cm), streamed: every half-tile split into 4 q1 bins, chunk flags in
+// a.ss.  Status -1 when the tile does not fit.
 template <int K, int W>
 static LaunchResult launch_tile_stream(const LaunchArgs& a) {
     const int M = a.op.n_q * K;
@@ -121,15 +129,9 @@ static LaunchResult launch_tile_stream(const LaunchArgs& a) {
     sc.bin_begin = a.bin_begin;
     sc.bin_q1 = a.bin_q1;
     sc.n_ht = (int)n_ht;
-    if (a.ss->ready) {
-        sc.n_whole = 0;
-        sc.split = 4;
-    } else {
-        const int64_t n_whole = n_ht > ctas ? n_ht - ctas : 0;
-        sc.n_whole = (int)n_whole;
-        sc.split = (n_ht - n_whole) * 4 >= ctas ? 4 : 16;
-    }
-    const int64_t n_units = sc.n_whole + (n_ht - sc.n_whole) * sc.split;
+    sc.n_whole = 0;
+    sc.split = 4;
+    const int64_t n_units = n_ht * sc.split;
     if (n_units > INT32_MAX) return {2, 0, cudaSuccess, PATH_TILE};
     sc.n_units = (int)n_units;
     sc.counter = a.counter;
@@ -215,9 +217,7 @@ static LaunchResult launch_outer(const LaunchArgs& a) {
         e = cudaMemsetAsync(a.counter, 0, sizeof(int), a.stream);
         if (e != cudaSuccess) return {5, 0, e, path};
     }
-    // few units: whole numbers of CTAs for each (L = 7, K = 8, 64 cells: J.v 47 against 68 us)
-    const int64_t most = !stream && ctas >= 8 * n_ht ? ctas / n_ht * n_ht : ctas;
-    const unsigned grid = (unsigned)std::min<int64_t>(stream ? cuts.n_units : n_ht * a.op.n_items, most);
+    const unsigned grid = stream ? (unsigned)std::min<int64_t>(cuts.n_units, ctas) : stretch_grid(a, n_ht, ctas);
     const StreamSync none{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, 0};
     kern<<<grid, kOuterWarps * 32, smem, a.stream>>>(a.op, sc, g, a.ss ? *a.ss : none, g.tiled ? a.fT : a.f_cm,
                                                     g.tiled ? a.vT : a.v_cm, g.tiled ? a.QT : a.q_cm,
@@ -233,11 +233,13 @@ static LaunchResult launch_pair(const LaunchArgs& a) {
                                        sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(K, JV));
     int share = 0;
     if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT) {
-        // a batch of fewer half-tiles than SMs: room behind the tile for the part sums of units with fewer
-        // items than warps (a larger one keeps its shared memory for a second CTA on the SM)
+        // a batch of fewer half-tiles than SMs: room behind the tile for the part sums of units with fewer items than
+        // warps, as far as the CTAs per SM stay the same (L = 12, K = 4, 2048 cells, plain: 1335 us with one CTA of
+        // 8 warps an SM and all parts shared, 1156 us with two CTAs)
         constexpr size_t per_item = sizeof(double) * kRowParts * K * 32;
-        if ((a.n_cells + kTileCells - 1) / kTileCells < a.n_sms && smem + 256 <= a.max_smem) {
-            share = (int)std::min<size_t>(W - 1, (a.max_smem - 256 - smem) / per_item);
+        const size_t room = (a.max_smem + 1024) / (K <= 4 && !RG && 2 * (smem + 1280) <= a.max_smem + 1024 ? 2 : 1) - 1024 - 256;
+        if ((a.n_cells + kTileCells - 1) / kTileCells < a.n_sms && smem <= room) {
+            share = (int)std::min<size_t>(W - 1, (room - smem) / per_item);
             smem += share * per_item;
         }
     }
@@ -250,9 +252,9 @@ static LaunchResult launch_pair(const LaunchArgs& a) {
     if (per_sm < 1) return {-1, 0, cudaSuccess, PATH_PAIR};
     const int64_t ctas = (int64_t)per_sm * a.n_sms;
     if ((a.n_cells + kTileCells - 1) / kTileCells * 16 > INT32_MAX) return {2, 0, cudaSuccess, PATH_PAIR};
-    // sixteenths where their few items are shared out by parts (L = 12, K = 5, 2048 cells: 958 against 1038 us;
+    // sixteenths where their few items (of two rows) are shared out by parts (L = 12, K = 5, 2048 cells: 958 against 1038 us;
     // unshared ones are slower: L = 8, K = 6, 4096 cells 887 against 811 us)
-    const UnitCuts cuts = cut_units((a.n_cells + kTileCells - 1) / kTileCells, ctas, share > 0);
+    const UnitCuts cuts = cut_units((a.n_cells + kTileCells - 1) / kTileCells, ctas, share * 32 >= a.op.n_items);
     PairSched sc{a.pbin_begin, a.pbin_item, a.pitems, cuts, a.counter, share};
     e = cudaMemsetAsync(a.counter, 0, sizeof(int), a.stream);
     if (e != cudaSuccess) return {5, 0, e, PATH_PAIR};
@@ -497,14 +499,15 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
     if (a.ss) {
         if (a.what == OP_RF || a.exact || a.f32) return {8, 0, cudaSuccess, PATH_TILE};
         if constexpr (outer_for(K)) {
-            if (a.path == PATH_AUTO && outer_takes(a.op.n_q, K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms)) {
+            if (a.path == PATH_AUTO && outer_takes(K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms)) {
                 const LaunchResult r = a.what == OP_JV ? launch_outer<K, true>(a) : launch_outer<K, false>(a);
                 if (r.status != -1) return r;
             }
         }
         if (a.what != OP_AF) return {8, 0, cudaSuccess, PATH_TILE};
         if constexpr (K % 2 == 0 && K <= 8) {
-            const LaunchResult r = launch_tile_stream<K, tile_W(K, false)>(a);
+            const LaunchResult r = a.ss->ready ? launch_tile_stream<K, tile_W(K, false)>(a)
+                                               : launch_tile<K, tile_W(K, false), false, false, true>(a);
             if (r.status == -1) return {8, 0, cudaSuccess, PATH_TILE};
             return r;
         } else {
@@ -560,7 +563,7 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
         return launch_for_k<K>(b);
     }
     if constexpr (outer_for(K)) {
-        if (a.path == PATH_AUTO && !a.exact && outer_takes(a.op.n_q, K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms)) {
+        if (a.path == PATH_AUTO && !a.exact && outer_takes(K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms)) {
             const LaunchResult r = jv ? launch_outer<K, true>(a) : launch_outer<K, false>(a);
             if (r.status != -1) return r;
         }
@@ -584,14 +587,14 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
             LaunchResult r;
             if (a.path == PATH_PAIR_L1) {
                 if (jv)
-                    r = a.exact ? launch_pair<K, pair_W(K, true), true, true, true>(a) : launch_pair<K, pair_W(K, true), false, true, true>(a);
+                    r = a.exact ? launch_pair<K, 8, true, true, true>(a) : launch_pair<K, pair_W(K, true), false, true, true>(a);
                 else
-                    r = a.exact ? launch_pair<K, pair_W(K), true, false, true>(a) : launch_pair<K, pair_W(K), false, false, true>(a);
+                    r = a.exact ? launch_pair<K, 8, true, false, true>(a) : launch_pair<K, pair_W(K), false, false, true>(a);
             } else {
                 if (jv)
-                    r = a.exact ? launch_pair<K, pair_W(K, true), true, true, false>(a) : launch_pair<K, pair_W(K, true), false, true, false>(a);
+                    r = a.exact ? launch_pair<K, 8, true, true, false>(a) : launch_pair<K, pair_W(K, true), false, true, false>(a);
                 else
-                    r = a.exact ? launch_pair<K, pair_W(K), true, false, false>(a) : launch_pair<K, pair_W(K), false, false, false>(a);
+                    r = a.exact ? launch_pair<K, 8, true, false, false>(a) : launch_pair<K, pair_W(K), false, false, false>(a);
             }
             if (r.status == -1 && a.path != PATH_PAIR_L1 && jv && !a.exact && pair_W(K, true) > 8)
                 r = launch_pair<K, 8, false, true, false>(a);  // fewer copies of R_t

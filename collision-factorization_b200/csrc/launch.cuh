@@ -97,15 +97,16 @@ constexpr bool pair_fits(int n_q, int K, bool jv, size_t max_smem) {
     return K <= 8 && sizeof(double) * ((size_t)(jv ? 2 : 1) * n_q * K * 16 + (size_t)pair_W(K, jv) * pair_warp_doubles(K, jv)) +
                              256 <= max_smem;
 }
+constexpr int kTileBufs = 4;  // half-tiles that a CTA of the tile kernel holds at a time, at most
 // K that the outer-product kernels (outer_kernels.cuh) take.
 constexpr bool outer_for(int K) { return K >= 7 && K <= 8; }
 
 // Where they are the faster family (B200, us, outer / tile or pair): nearly everywhere (folded Q, K = 8: L = 10, 4096
 // cells 1509 / 1642, L = 13, 1000 cells 1045 / 1928, L = 6, 2048 cells 161 / 176, L = 3, 2000 cells 39 / 51; J.v, L = 10,
-// 2174 / 3060; plain Q, K = 7, L = 5, 4096 cells 250 / 266).  The pair kernel keeps the plain J.v at K = 7 below L = 7
-// (L = 4, 4000 cells: 189 / 176; L = 6, 2000 cells: 312 / 299) unless the batch has at most half a half-tile per SM.
-constexpr bool outer_takes(int n_q, int K, bool folded, bool jv, int64_t n_cells, int n_sms) {
-    return outer_for(K) && (K == 8 || folded || !jv || n_q >= 64 || (n_cells + 15) / 16 * 2 <= n_sms);
+// 2174 / 3060; plain Q, K = 7, L = 5, 4096 cells 250 / 266).  The pair kernel keeps the plain J.v at K = 7 on batches of more
+// than two thirds of a half-tile per SM (L = 8: 4096 cells 1677 / 1570, 1300 cells 571 / 691; L = 6, 2000 cells: 312 / 299).
+constexpr bool outer_takes(int K, bool folded, bool jv, int64_t n_cells, int n_sms) {
+    return outer_for(K) && (K == 8 || folded || !jv || (n_cells + 15) / 16 * 3 <= 2 * n_sms);
 }
 
 // Shared-memory geometry of the outer-product kernels.  Cells lie in pairs, [pair][k][q][cell of the pair],

@@ -32,7 +32,7 @@
 namespace cf {
 
 // Work of one launch.  The units' rows, heaviest first, unit after unit, are one list that the CTAs share out in
-// contiguous stretches of equal work (x_cum): at most two cut units a CTA, so teams run out of rows twice and f is
+// contiguous stretches of equal work (item_cum): at most two cut units a CTA, so teams run out of rows twice and f is
 // staged little more than once.  Against whole units, then quarters, then sixteenths from a counter (B200, us):
 // folded K = 8: L = 10, 4096 cells 1542 -> 1509, 300 cells 193 -> 158; L = 8, 2048 cells: J.v 543 -> 502; L = 13, 1000
 // cells: 1120 -> 1045.  A streamed launch keeps quarters in order of arrival, so that every chunk gives work to all CTAs.
@@ -291,16 +291,8 @@ __global__ void __launch_bounds__(kOuterWarps * 32, 1)
     // not streamed: what is left of this CTA's stretch, from row s_from.y of unit s_from.x to row s_to.y of unit s_to.x
     __shared__ int2 s_from, s_to;
     if (!ss.ready) {
-        const int n = op.n_items;  // <= N_Q <= 268 < the CTA's threads
-        const long long total = op.x_cum[n], work = total * sc.cuts.n_four;
-        // the row boundary nearest to a place in the list
-        auto cut = [&](int i) {
-            const long long at = work * i / gridDim.x;
-            const int u = (int)(at / total), rem = (int)(at - u * total);
-            const int r = __syncthreads_count(tid < n && op.x_cum[tid] + op.x_cum[min(tid, n - 1) + 1] <= 2 * rem);
-            return r == n ? make_int2(u + 1, 0) : make_int2(u, r);
-        };
-        const int2 from = cut(blockIdx.x), to = cut(blockIdx.x + 1);
+        const int2 from = stretch_cut<W * 32>(op, sc.cuts.n_four, blockIdx.x),
+                   to = stretch_cut<W * 32>(op, sc.cuts.n_four, blockIdx.x + 1);
         if (tid == 0) {
             s_from = from;
             s_to = to;

@@ -74,6 +74,7 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
     const int q1 = half == 0 ? item.x : (item.y >= 0 ? item.y : item.x);
 
     constexpr bool PARTS = F64 && !EXACT;
+    constexpr bool AHEAD = F64 && !EXACT && K > 4;  // below, and in the exact and FP32 forms, 2 % slower
     T acc[K];
     double tot[PARTS && !TS ? K : 1];
     double* ts = TS ? reinterpret_cast<double*>(rb) + RPair<K, T>::SIZE + lane : nullptr;
@@ -121,7 +122,7 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
     int g_end = i_hi, g_no = 0;  // end and number of the part in work
     if constexpr (PARTS)
         if (part < 0) g_end = row_part(n_s, 1);
-    if (i_lo < i_hi) {
+    if (AHEAD && i_lo < i_hi) {
         range(i_lo);
         entries();
     }
@@ -141,10 +142,11 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
                     g_end = row_part(n_s, g_no + 1);
                 }
         }
+        if constexpr (!AHEAD) range(i);
         const int t = nx_t, n_e = nx_n, my_e0 = nx_e0;
         const uint32_t q23_0 = nx_q23;
         const double g_0 = nx_g;
-        if (i + 1 < i_hi) range(i + 1);
+        if (AHEAD && i + 1 < i_hi) range(i + 1);
 
         const T* __restrict__ Rt = r_tensor<T>(op) + (size_t)t * K * K * K;
         if constexpr (RG) {
@@ -174,7 +176,7 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
             const int n = min(16, n_e - e0);
             uint32_t my_q23 = q23_0;
             double my_g = g_0;
-            if (e0 > 0) {
+            if (!AHEAD || e0 > 0) {
                 my_q23 = 0;
                 my_g = 0.0;
                 if (c < n && active) {
@@ -233,7 +235,7 @@ __device__ __forceinline__ void pair_item(const DevOp& op, int2 item, const T* _
                 }
             }
         }
-        if (i + 1 < i_hi) entries();
+        if (AHEAD && i + 1 < i_hi) entries();
         if constexpr (!RG) {
             cp_async_wait_all();
             __syncwarp();
@@ -487,7 +489,8 @@ __device__ __forceinline__ void pair_split_item(const DevOp& op, int2 item, cons
 
 // fT, vT: tiled cells in T (FP64 tiles for the FP64 forms, FP32 tiles for the FP32 form); QT: FP64.
 // CM: fT, vT, QT are the caller's cell-major arrays of n_cells cells (FP64 forms).  sc.share: where a unit has
-// fewer items than warps, the warps take its (item, part) pairs and the parts are added from shared memory.
+// fewer items than warps, the warps take (item, part) pairs, of that many items at a time, and the parts are added from
+// shared memory.
 template <int K, int W, bool EXACT, bool JV, bool RG, typename T = double, bool SPLIT = false, bool CM = false>
 __global__ void __launch_bounds__(W * 32, sizeof(T) == 8 && K <= 4 && !RG ? 2 : 1)
     af_pair_kernel(DevOp op, PairSched sc, const T* __restrict__ fT, const T* __restrict__ vT,
@@ -543,35 +546,41 @@ __global__ void __launch_bounds__(W * 32, sizeof(T) == 8 && K <= 4 && !RG ? 2 : 
         const bool live = !CM || cell0 + (lane & 15) < n_cells;
         double* qtc = CM ? QT + (size_t)(live ? cell0 + (lane & 15) : 0) * M : QT + tile_base + (lane & 15);
         if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT) {
-            if (nb < W && nb <= sc.share) {
-                // part sums [item][part][k1][lane] behind the warps' R buffers
+            if (nb < W && (nb <= sc.share || 4 * sc.share >= W)) {
+                // up to sc.share items at a time, in even groups (fewer than a quarter of the warps would leave warps idle: L = 16,
+                // K = 5, 64 cells 506 against 380 us): part sums [item][part][k1][lane] behind the warps' R buffers
                 double* parts = reinterpret_cast<double*>(smem) + (size_t)(JV ? 2 : 1) * M * kTileCells +
                                 (RG ? 0 : (size_t)W * WB);
-                for (;;) {
-                    int i = 0;
-                    if (lane == 0) i = atomicAdd(&s_next, 1);
-                    i = __shfl_sync(0xffffffffu, i, 0);
-                    if (i >= nb * kRowParts) break;
-                    double sum[K];
-                    pair_item<K, EXACT, JV, RG, T, CM, TS>(op, sc.items[sc.bin_item[b0 + i / kRowParts]], fs, vs, rb, qtc,
-                                                       lane, live, i % kRowParts, sum);
+                const int groups = (nb + sc.share - 1) / sc.share, size = (nb + groups - 1) / groups;
+                for (int g0 = 0; g0 < nb; g0 += size) {
+                    const int ng = min(size, nb - g0);
+                    for (;;) {
+                        int i = 0;
+                        if (lane == 0) i = atomicAdd(&s_next, 1);
+                        i = __shfl_sync(0xffffffffu, i, 0);
+                        if (i >= ng * kRowParts) break;
+                        double sum[K];
+                        pair_item<K, EXACT, JV, RG, T, CM, TS>(op, sc.items[sc.bin_item[b0 + g0 + i / kRowParts]], fs, vs,
+                                                           rb, qtc, lane, live, i % kRowParts, sum);
 #pragma unroll
-                    for (int k1 = 0; k1 < K; ++k1) parts[(i * K + k1) * 32 + lane] = sum[k1];
-                }
-                __syncthreads();
-                for (int i = warp; i < nb; i += W) {
-                    const int2 it = sc.items[sc.bin_item[b0 + i]];
-                    const int q1 = lane < 16 ? it.x : it.y;
-                    if (q1 < 0 || !live) continue;
-#pragma unroll
-                    for (int k1 = 0; k1 < K; ++k1) {
-                        double* out = qtc + q_off<K, CM>(q1, k1, op.n_q);
-                        double x = *out;
-                        for (int g = 0; g < kRowParts; ++g) x += parts[((i * kRowParts + g) * K + k1) * 32 + lane];
-                        *out = x;
+                        for (int k1 = 0; k1 < K; ++k1) parts[(i * K + k1) * 32 + lane] = sum[k1];
                     }
+                    __syncthreads();
+                    if (tid == 0) s_next = 0;
+                    for (int i = warp; i < ng; i += W) {
+                        const int2 it = sc.items[sc.bin_item[b0 + g0 + i]];
+                        const int q1 = lane < 16 ? it.x : it.y;
+                        if (q1 < 0 || !live) continue;
+#pragma unroll
+                        for (int k1 = 0; k1 < K; ++k1) {
+                            double* out = qtc + q_off<K, CM>(q1, k1, op.n_q);
+                            double x = *out;
+                            for (int g = 0; g < kRowParts; ++g) x += parts[((i * kRowParts + g) * K + k1) * 32 + lane];
+                            *out = x;
+                        }
+                    }
+                    __syncthreads();
                 }
-                __syncthreads();
                 continue;
             }
         }

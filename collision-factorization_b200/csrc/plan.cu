@@ -105,11 +105,11 @@ struct cf_plan {
     double* d_RT = nullptr;  // K = 8: R_t as [k1][8 k2 + k3] for the MMA kernel
     unsigned short* d_RTbf = nullptr;  // K = 8: the same split into BF16 hi and lo parts
     int* d_x_q1 = nullptr;
-    int* d_x_cum = nullptr;
     int4* d_x_slice = nullptr;  // outer-product kernels' tables (build_outer)
     unsigned char* d_x_chunk = nullptr;
     double2* d_x_R = nullptr;
     int* d_item_q1 = nullptr;
+    long long* d_item_cum = nullptr;
     int* d_bin_begin = nullptr;  // q1 bins of the tile kernel's work units (bin 0 = all, 1..4, 5..20)
     int* d_bin_q1 = nullptr;
     // work-queue heads of the persistent kernels: one slot per stream (kCounterSlots slots, assigned
@@ -182,7 +182,7 @@ struct cf_plan {
         o.RT = d_RT;
         o.RTbf = d_RTbf;
         o.x_q1 = d_x_q1;
-        o.x_cum = d_x_cum;
+        o.item_cum = d_item_cum;
         o.x_slice = d_x_slice;
         o.x_chunk = d_x_chunk;
         o.x_R = d_x_R;
@@ -285,7 +285,7 @@ void free_plan_memory(cf_plan* p) {
     cudaFree(p->d_RT);
     cudaFree(p->d_RTbf);
     cudaFree(p->d_x_q1);
-    cudaFree(p->d_x_cum);
+    cudaFree(p->d_item_cum);
     cudaFree(p->d_x_slice);
     cudaFree(p->d_x_chunk);
     cudaFree(p->d_x_R);
@@ -319,7 +319,7 @@ void free_plan_memory(cf_plan* p) {
 // in the list's own order).
 int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<int>& slice_t,
                 const std::vector<int>& slice_e, const std::vector<uint32_t>& e_q23, const std::vector<double>& e_g,
-                const std::vector<int>& items, int64_t& bytes) {
+                int64_t& bytes) {
     constexpr size_t kLook = 6;  // candidates per place
     struct Run {
         unsigned short q2, qa, qb, two;
@@ -409,14 +409,6 @@ int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<
     }
     for (size_t q = 0; q < q1_begin.size(); ++q) xq1[q] = xbegin[q1_begin[q]];
     CF_TRY(upload(&p->d_x_q1, xq1, bytes));
-    // the rows' work added up in list order: a slice (R_t, ring) about 4/3 of a chunk, a row's end 2
-    std::vector<int> xcum(1, 0);
-    for (int q : items) {
-        int w = 6;
-        for (int s = xq1[q]; s < xq1[q + 1]; ++s) w += 4 + 3 * xs[s].w;
-        xcum.push_back(xcum.back() + w);
-    }
-    CF_TRY(upload(&p->d_x_cum, xcum, bytes));
     CF_TRY(upload(&p->d_x_slice, xs, bytes));
     CF_TRY(upload(&p->d_x_chunk, xb, bytes));
     const size_t nR = (size_t)p->n_l * p->k * 32;
@@ -571,6 +563,12 @@ int build_plan(cf_plan* p, const double* labels, const double* vals, const doubl
         }
     }
     CF_TRY(upload(&p->d_item_q1, items, bytes));
+    // the rows' work in list order, added up: an entry K^2 FMAs, a slice K^3, a row's end about as much
+    std::vector<long long> item_cum(1, 0);
+    for (int q : items)
+        item_cum.push_back(item_cum.back() + (long long)(q1_begin[q + 1] - q1_begin[q] + 1) * K +
+                           slice_e[q1_begin[q + 1]] - slice_e[q1_begin[q]]);
+    CF_TRY(upload(&p->d_item_cum, item_cum, bytes));
     CF_TRY(upload(&p->d_bin_begin, bin_begin, bytes));
     CF_TRY(upload(&p->d_bin_q1, bin_q1, bytes));
     CF_TRY(upload(&p->d_pbin_begin, pbin_begin, bytes));
@@ -584,7 +582,7 @@ int build_plan(cf_plan* p, const double* labels, const double* vals, const doubl
     CF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     p->max_smem = (size_t)optin;
     if (cf::outer_for(K) && cf::outer_fit(NQ, K, false, p->max_smem).nc > 0)
-        CF_TRY(build_outer(p, q1_begin, slice_t, slice_e, e_q23, e_g, items, bytes));
+        CF_TRY(build_outer(p, q1_begin, slice_t, slice_e, e_q23, e_g, bytes));
     CF_CUDA(cudaStreamSynchronize(nullptr));  // a launch on another stream may read what the kernels here wrote
     p->dev_bytes = bytes;
     return CF_OK;
@@ -773,7 +771,7 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
     if (ws_bytes < need) return fail(CF_EINVAL, "workspace of %zu bytes is smaller than %zu", ws_bytes, need);
     // The fast FP64 Q and J.v forms on the outer-product kernel: one launch on the cell-major arrays.
     if (!exact && f32 == 0 && (what == 0 || what == 2) && p->path == cf::PATH_AUTO &&
-        cf::outer_takes(p->n_q, p->k, sym, what == 2, B, p->n_sms) &&
+        cf::outer_takes(p->k, sym, what == 2, B, p->n_sms) &&
         cf::outer_fit(p->n_q, p->k, what == 2, p->max_smem).nc > 0) {
         cf_plan* target = p;
         if (sym) CF_TRY(get_sym(p, &target));

@@ -9,12 +9,12 @@
 //   * per (t, q1) slice the warp copies R_t into its own shared buffer with cp.async while it
 //     accumulates Phi, so the K^3 step reads R from shared memory (k3 slices padded by two doubles
 //     so the two lane halves hit different banks);
-//   * CTAs are persistent and pull work units from a device counter: whole half-tiles first, then
-//     half-tiles split into q1 bins, so the last wave is made of small units.  Inside a unit the
+//   * a CTA takes an equal share of all rows of all half-tiles (af_tile_kernel) or, in the kernels that still
+//     pull units from a device counter, whole half-tiles and then parts of the last ones.  Inside, the
 //     warps pull q1 values (heaviest first) from a shared counter.
 //
-// The counter is the only inter-CTA interaction; nothing waits on another CTA.  The streamed
-// variant at the end also waits, with a bound, on flags that the host's copies set.
+// Nothing waits on another CTA.  The streamed
+// variant at the end waits, with a bound, on flags that the host's copies set.
 #pragma once
 #include "common.cuh"
 
@@ -68,6 +68,22 @@ struct RBuf {
     static constexpr int SIZE = K * SL;
 };
 
+// The place in the list of all units' rows (item_q1, unit after unit) that is nearest to i / gridDim.x of its work, as
+// (unit, row).  All T threads of the CTA call it.
+template <int T>
+__device__ __forceinline__ int2 stretch_cut(const DevOp& op, int n_units, int i) {
+    const int n = op.n_items;
+    const long long total = op.item_cum[n], at = total * n_units / gridDim.x * i + total * n_units % gridDim.x * i / gridDim.x;
+    const int u = (int)(at / total);
+    const long long rem = at - u * total;
+    int r = 0;
+    for (int b = 0; b < n; b += T) {
+        const int j = b + (int)threadIdx.x;
+        r += __syncthreads_count(j < n && op.item_cum[min(j, n - 1)] + op.item_cum[min(j, n - 1) + 1] <= 2 * rem);
+    }
+    return r == n ? make_int2(u + 1, 0) : make_int2(u, r);
+}
+
 // Offset of Q[q1][k1] from a lane's cell: tiled rows (stride CF_TILE) or, with CELL_MAJOR, the
 // caller's [N_Q x K x B] layout (qtc then points at the cell's first element).
 template <int K, bool CELL_MAJOR>
@@ -75,12 +91,13 @@ __device__ __forceinline__ size_t q_off(int q1, int k1, int n_q) {
     return CELL_MAJOR ? (size_t)q1 + (size_t)k1 * n_q : (size_t)(q1 * K + k1) * CF_TILE;
 }
 
-// Stage a half-tile from the caller's cell-major array: element j = q + N_Q k of cell c goes to row q K + k;
-// a warp reads two consecutive j of 16 cells and writes two 16-cell rows of shared memory.
+// Stage a half-tile from the caller's cell-major array: element j = q + N_Q k of cell c goes to row q K + k.
 template <int K>
 __device__ __forceinline__ void stage_cells(double* fs, const double* __restrict__ f, int n_q, long long cell0,
                                             long long n_cells, int tid, int threads) {
     const int M = n_q * K;
+    // a warp: two neighbouring elements of 16 cells (four of eight, whole sectors, write 4-way conflicts: 465 against 436 us
+    // at L = 8, K = 4, 4096 cells, plain)
     for (int i = tid; i < M * kTileCells; i += threads) {
         const int c = i & 15, j = i >> 4;
         const int r = (j % n_q) * K + j / n_q;
@@ -302,71 +319,76 @@ __device__ __forceinline__ void tile_q1(const DevOp& op, int q1, const double* _
     }
 }
 
-template <int K, int W, bool EXACT, bool JV>
+// The rows of all half-tiles, heaviest first, half-tile after half-tile, are one list that the CTAs share out in
+// contiguous stretches of equal work.  Up to n_buf half-tiles of a stretch are resident at a time and their rows,
+// last half-tile first (its rows are the heavy ones), are one list for the CTA's warps: a stretch ends in one
+// partly filled round of rows, not one per half-tile, and f is read once or twice.  Against whole half-tiles, then
+// quarters, then sixteenths from a counter (B200, folded, us): L = 6, K = 6: 2048 cells 119 -> 95,
+// 500 cells 84 -> 37; L = 8, K = 6, 4096 cells 518 -> 447; L = 4, K = 4, 4000 cells 51 -> 35; J.v L = 10, K = 6, 2000
+// cells 908 -> 835.
+template <int K, int W, bool EXACT, bool JV, bool CM>
 __global__ void __launch_bounds__(W * 32, 1)
-    af_tile_kernel(DevOp op, TileSched sc, const double* __restrict__ fT, const double* __restrict__ vT,
-                   double* __restrict__ QT) {
+    af_tile_kernel(DevOp op, int n_ht, int n_buf, const double* __restrict__ f, const double* __restrict__ v,
+                   double* __restrict__ q, long long n_cells) {
     static_assert(K % 2 == 0, "the tile kernel splits Phi into two column halves");
     extern __shared__ __align__(16) double smem[];
-    __shared__ int s_unit, s_next;
+    __shared__ int s_next;
     const int M = op.n_q * K;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    double* fs = smem;
-    double* vs = JV ? smem + (size_t)M * kTileCells : nullptr;
-    double* rb = smem + (size_t)(JV ? 2 : 1) * M * kTileCells + (size_t)warp * RBuf<K>::SIZE;
-    int staged = -1;
+    const int one = M * kTileCells, tile = (JV ? 2 : 1) * one;  // elements of a resident array, of a half-tile
+    double* rb = smem + (size_t)n_buf * tile + (size_t)warp * RBuf<K>::SIZE;
+    const int2 from = stretch_cut<W * 32>(op, n_ht, blockIdx.x), to = stretch_cut<W * 32>(op, n_ht, blockIdx.x + 1);
+    const int last = to.y > 0 ? to.x : to.x - 1;
 
-    for (;;) {
-        if (tid == 0) s_unit = atomicAdd(sc.counter, 1);
-        __syncthreads();
-        const int u = s_unit;
-        if (u >= sc.n_units) break;
-        int ht, bin;
-        if (u < sc.n_whole) {
-            ht = u;
-            bin = 0;
-        } else {
-            const int v = u - sc.n_whole;
-            ht = sc.n_whole + v / sc.split;
-            bin = bin_base(sc.split) + v % sc.split;
-        }
-        const size_t tile_base = (size_t)(ht >> 1) * M * CF_TILE + (size_t)(ht & 1) * kTileCells;
-        if (ht != staged) {
-            // rows of 16 cells (128 B) from the tiled global layout, 8 x 16-byte copies per row
-            const double* srcf = fT + tile_base;
-            for (int i = tid; i < M * 8; i += W * 32) {
-                const int r = i >> 3, w = (i & 7) * 2;
-                cp_async16(fs + r * kTileCells + w, srcf + (size_t)r * CF_TILE + w);
-            }
-            if constexpr (JV) {
-                const double* srcv = vT + tile_base;
+    for (int h0 = from.x; h0 <= last; h0 += n_buf) {
+        const int n = min(n_buf, last - h0 + 1);
+        for (int h = 0; h < n; ++h) {
+            const int ht = h0 + h;
+            double* fs = smem + (size_t)h * tile;
+            if constexpr (CM) {
+                stage_cells<K>(fs, f, op.n_q, (long long)ht * kTileCells, n_cells, tid, W * 32);
+                if constexpr (JV) stage_cells<K>(fs + one, v, op.n_q, (long long)ht * kTileCells, n_cells, tid, W * 32);
+            } else {
+                // rows of 16 cells (128 B) from the tiled global layout, 8 x 16-byte copies per row
+                const size_t base = (size_t)(ht >> 1) * M * CF_TILE + (size_t)(ht & 1) * kTileCells;
                 for (int i = tid; i < M * 8; i += W * 32) {
                     const int r = i >> 3, w = (i & 7) * 2;
-                    cp_async16(vs + r * kTileCells + w, srcv + (size_t)r * CF_TILE + w);
+                    cp_async16(fs + r * kTileCells + w, f + base + (size_t)r * CF_TILE + w);
+                    if constexpr (JV) cp_async16(fs + one + r * kTileCells + w, v + base + (size_t)r * CF_TILE + w);
                 }
             }
-            cp_async_commit();
-            cp_async_wait_all();
-            staged = ht;
         }
+        cp_async_commit();
+        cp_async_wait_all();
         if (tid == 0) s_next = 0;
         __syncthreads();
-        const int b0 = sc.bin_begin[bin], nb = sc.bin_begin[bin + 1] - b0;
-        double* qtc = QT + tile_base + (lane & 15);
         for (;;) {
             int i = 0;
             if (lane == 0) i = atomicAdd(&s_next, 1);
             i = __shfl_sync(0xffffffffu, i, 0);
-            if (i >= nb) break;
-            tile_q1<K, EXACT, JV>(op, sc.bin_q1[b0 + i], fs, vs, rb, qtc, lane);
+            int h = n - 1, lo = 0;
+            for (; h >= 0; --h) {
+                lo = h0 + h == from.x ? from.y : 0;
+                const int rows = (h0 + h == to.x ? to.y : op.n_items) - lo;
+                if (i < rows) break;
+                i -= rows;
+            }
+            if (h < 0) break;
+            const int ht = h0 + h;
+            const long long cell = (long long)ht * kTileCells + (lane & 15);
+            const bool live = !CM || cell < n_cells;
+            double* qc = CM ? q + (size_t)(live ? cell : 0) * M
+                            : q + (size_t)(ht >> 1) * M * CF_TILE + (size_t)(ht & 1) * kTileCells + (lane & 15);
+            const double* fs = smem + (size_t)h * tile;
+            tile_q1<K, EXACT, JV, CM>(op, op.item_q1[lo + i], fs, fs + one, rb, qc, lane, live);
         }
         __syncthreads();
     }
 }
 
 template <int K>
-constexpr size_t tile_smem_bytes(int M, int W, bool jv) {
-    return sizeof(double) * ((size_t)(jv ? 2 : 1) * M * kTileCells + (size_t)W * RBuf<K>::SIZE);
+constexpr size_t tile_smem_bytes(int M, int W, bool jv, int n_buf = 1) {
+    return sizeof(double) * ((size_t)n_buf * (jv ? 2 : 1) * M * kTileCells + (size_t)W * RBuf<K>::SIZE);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -573,8 +595,7 @@ constexpr size_t tile4_smem_bytes(int M, int W, bool jv) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Tile kernel on the caller's cell-major f and Q.  Resident (ss.ready == null): the device entry
-// points, no layout passes, the tile kernel's schedule.  Streamed (host entry points): one launch
+// Tile kernel on the caller's cell-major f and Q, streamed (host entry points): one launch
 // over the whole batch while the batch is still being copied in and the results copied out.
 //
 // f and Q stay in the caller's cell-major layout [N_Q x K x B] in device memory.  The host cuts
@@ -614,19 +635,11 @@ __global__ void __launch_bounds__(W * 32, 1)
         __syncthreads();
         const int u = s_unit;
         if (u >= sc.n_units) break;
-        int ht, bin;
-        if (u < sc.n_whole) {
-            ht = u;
-            bin = 0;
-        } else {
-            const int v = u - sc.n_whole;
-            ht = sc.n_whole + v / sc.split;
-            bin = bin_base(sc.split) + v % sc.split;
-        }
+        const int ht = u / sc.split, bin = bin_base(sc.split) + u % sc.split;
         const int chunk = ht / ss.ht_per_chunk;
         const long long cell0 = (long long)ht * kTileCells;
         if (ht != staged) {
-            if (tid == 0 && ss.ready) {
+            if (tid == 0) {
                 const long long t0 = clock64();
                 while (ld_acquire(ss.ready + chunk) != ss.epoch) {
                     if (*reinterpret_cast<volatile int*>(ss.abort) == ss.epoch) break;
@@ -657,14 +670,10 @@ __global__ void __launch_bounds__(W * 32, 1)
             if (i >= nb) break;
             tile_q1<K, false, false, true>(op, sc.bin_q1[b0 + i], fs, nullptr, rb, qc, lane, live);
         }
-        if (ss.done) __threadfence();
+        __threadfence();
         __syncthreads();
-        if (tid == 0 && ss.done) {
-            // units of this chunk: its half-tiles below n_whole are one unit each, the rest `split`
-            const int h0 = chunk * ss.ht_per_chunk;
-            const int c_ht = min(ss.ht_per_chunk, sc.n_ht - h0);
-            const int c_whole = max(0, min(c_ht, sc.n_whole - h0));
-            const int c_units = c_whole + (c_ht - c_whole) * sc.split;
+        if (tid == 0) {
+            const int c_units = min(ss.ht_per_chunk, sc.n_ht - chunk * ss.ht_per_chunk) * sc.split;
             if (atomicAdd(ss.done + chunk, 1) == c_units - 1) {
                 __threadfence_system();
                 *reinterpret_cast<volatile int*>(ss.host_done + chunk) = ss.epoch;

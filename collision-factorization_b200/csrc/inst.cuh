@@ -71,8 +71,8 @@ static LaunchResult launch_af(const LaunchArgs& a) {
 // CTAs of a launch whose rows are shared out in stretches (stretch_cut).  Few units: whole numbers of CTAs for each
 // (L = 7, K = 8, 64 cells: J.v 47 against 68 us), as a stretch of little more than a row should not take one row
 // from each of two units.
-static inline unsigned stretch_grid(const LaunchArgs& a, int64_t n_units, int64_t ctas) {
-    return (unsigned)std::min<int64_t>(n_units * a.op.n_items, ctas >= 8 * n_units ? ctas / n_units * n_units : ctas);
+static inline unsigned stretch_grid(int64_t n_rows, int64_t n_units, int64_t ctas) {
+    return (unsigned)std::min<int64_t>(n_units * n_rows, ctas >= 8 * n_units ? ctas / n_units * n_units : ctas);
 }
 
 // Tile-resident persistent kernel.  Returns status -1 when it does not fit (shared memory or
@@ -89,7 +89,7 @@ static LaunchResult launch_tile(const LaunchArgs& a) {
     if (per_sm < 1) return {-1, 0, cudaSuccess, PATH_TILE};
     const int64_t n_ht = (a.n_cells + kTileCells - 1) / kTileCells;
     if (n_ht > INT32_MAX / 16) return {2, 0, cudaSuccess, PATH_TILE};
-    const unsigned grid = stretch_grid(a, n_ht, (int64_t)per_sm * a.n_sms);
+    const unsigned grid = stretch_grid(a.op.n_items, n_ht, (int64_t)per_sm * a.n_sms);
     // as many half-tiles of a stretch at a time as fit beside each other, without an SM losing a CTA
     int n_buf = (int)std::min<int64_t>(kTileBufs, (n_ht + grid - 1) / grid + 1);
     while (n_buf > 1) {
@@ -211,13 +211,12 @@ static LaunchResult launch_outer(const LaunchArgs& a) {
     const int64_t n_ht = (a.n_cells + g.nc - 1) / g.nc;
     if (n_ht > INT32_MAX / 16) return {2, 0, cudaSuccess, path};
     // streamed: every half-tile in 4, so that the first chunk gives work to every CTA
-    const UnitCuts cuts{0, (int)n_ht, (int)n_ht * 4};
-    const OuterSched sc{a.bin_begin, a.bin_q1, cuts, a.counter};
+    const OuterSched sc{a.bin_begin, a.bin_q1, (int)n_ht, a.counter};
     if (stream) {
         e = cudaMemsetAsync(a.counter, 0, sizeof(int), a.stream);
         if (e != cudaSuccess) return {5, 0, e, path};
     }
-    const unsigned grid = stream ? (unsigned)std::min<int64_t>(cuts.n_units, ctas) : stretch_grid(a, n_ht, ctas);
+    const unsigned grid = stream ? (unsigned)std::min<int64_t>(n_ht * 4, ctas) : stretch_grid(a.op.n_items, n_ht, ctas);
     const StreamSync none{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, 0};
     kern<<<grid, kOuterWarps * 32, smem, a.stream>>>(a.op, sc, g, a.ss ? *a.ss : none, g.tiled ? a.fT : a.f_cm,
                                                     g.tiled ? a.vT : a.v_cm, g.tiled ? a.QT : a.q_cm,
@@ -229,36 +228,35 @@ static LaunchResult launch_outer(const LaunchArgs& a) {
 template <int K, int W, bool EXACT, bool JV, bool RG, typename T = double, bool SPLIT = false, bool CM = false>
 static LaunchResult launch_pair(const LaunchArgs& a) {
     const int M = a.op.n_q * K;
-    size_t smem = pair_smem_bytes<K, T>(M, W, JV, RG,
-                                       sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(K, JV));
-    int share = 0;
-    if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT) {
-        // a batch of fewer half-tiles than SMs: room behind the tile for the part sums of units with fewer items than
-        // warps, as far as the CTAs per SM stay the same (L = 12, K = 4, 2048 cells, plain: 1335 us with one CTA of
-        // 8 warps an SM and all parts shared, 1156 us with two CTAs)
-        constexpr size_t per_item = sizeof(double) * kRowParts * K * 32;
-        const size_t room = (a.max_smem + 1024) / (K <= 4 && !RG && 2 * (smem + 1280) <= a.max_smem + 1024 ? 2 : 1) - 1024 - 256;
-        if ((a.n_cells + kTileCells - 1) / kTileCells < a.n_sms && smem <= room) {
-            share = (int)std::min<size_t>(W - 1, (room - smem) / per_item);
-            smem += share * per_item;
-        }
-    }
-    if (smem + 256 > a.max_smem || a.counter == nullptr || a.pitems == nullptr) return {-1, 0, cudaSuccess, PATH_PAIR};
+    constexpr bool SUMS = sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(K, JV);
+    size_t smem = pair_smem_bytes<K, T>(M, W, JV, RG, SUMS);
+    if (smem + 256 > a.max_smem || a.n_pitems == 0) return {-1, 0, cudaSuccess, PATH_PAIR};
     static_assert(!SPLIT || (!EXACT && !JV && !RG && K % 2 == 0), "the split variant is the fast Q form");
     auto kern = af_pair_kernel<K, W, EXACT, JV, RG, T, SPLIT, CM>;
     int per_sm = 0;
     cudaError_t e = resident_ctas((const void*)kern, W * 32, smem, &per_sm);
     if (e != cudaSuccess) return {5, 0, e, PATH_PAIR};
     if (per_sm < 1) return {-1, 0, cudaSuccess, PATH_PAIR};
-    const int64_t ctas = (int64_t)per_sm * a.n_sms;
-    if ((a.n_cells + kTileCells - 1) / kTileCells * 16 > INT32_MAX) return {2, 0, cudaSuccess, PATH_PAIR};
-    // sixteenths where their few items (of two rows) are shared out by parts (L = 12, K = 5, 2048 cells: 958 against 1038 us;
-    // unshared ones are slower: L = 8, K = 6, 4096 cells 887 against 811 us)
-    const UnitCuts cuts = cut_units((a.n_cells + kTileCells - 1) / kTileCells, ctas, share * 32 >= a.op.n_items);
-    PairSched sc{a.pbin_begin, a.pbin_item, a.pitems, cuts, a.counter, share};
-    e = cudaMemsetAsync(a.counter, 0, sizeof(int), a.stream);
+    const int64_t n_ht = (a.n_cells + kTileCells - 1) / kTileCells;
+    if (n_ht > INT32_MAX / 16) return {2, 0, cudaSuccess, PATH_PAIR};
+    PairSched sc{a.pbin_item, a.pair_cum, a.pitems, a.n_pitems, (int)n_ht, 1, 0};
+    const unsigned grid = stretch_grid(sc.n_items, n_ht, (int64_t)per_sm * a.n_sms);
+    // room for part sums, then for more of the stretch's half-tiles, as far as the CTAs per SM stay the same (L = 12,
+    // K = 4, 2048 cells, plain: 1335 us with one CTA of 8 warps an SM and all parts shared, 1156 us with two CTAs)
+    const size_t room = (a.max_smem + 1024) / per_sm - 1024 - 256;
+    if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT) {
+        constexpr size_t per_item = sizeof(double) * kRowParts * K * 32;
+        if (smem < room) sc.share = (int)std::min<size_t>(W - 1, (room - smem) / per_item);
+        smem += sc.share * per_item;
+    }
+    const size_t tile = pair_smem_bytes<K, T>(M, W, JV, RG, SUMS, 2) - pair_smem_bytes<K, T>(M, W, JV, RG, SUMS);
+    while (sc.n_buf < kTileBufs && sc.n_buf < (n_ht + grid - 1) / grid + 1 && smem + tile <= room) {
+        smem += tile;
+        ++sc.n_buf;
+    }
+    e = resident_ctas((const void*)kern, W * 32, smem, &per_sm);
     if (e != cudaSuccess) return {5, 0, e, PATH_PAIR};
-    const unsigned grid = (unsigned)std::min<int64_t>(cuts.n_units, ctas);
+    if (per_sm < 1) return {-1, 0, cudaSuccess, PATH_PAIR};
     const T* fT;
     const T* vT;
     if constexpr (CM) {

@@ -39,9 +39,10 @@ struct LaunchArgs {
     int n_sms;
     size_t max_smem;
     // pair kernels: bins over pair items, items (qa, qb)
-    const int* pbin_begin;
     const int* pbin_item;
     const int2* pitems;
+    const long long* pair_cum;  // [n_pitems + 1] work of the items pbin_item[0 .. i) added up
+    int n_pitems;
     // FP32 form: tiled FP32 copies of f (and v) in place of fT / vT
     bool f32;
     const float* fT32;

@@ -39,7 +39,7 @@ namespace cf {
 struct OuterSched {
     const int* bin_begin;  // as TileSched (streamed)
     const int* bin_q1;
-    UnitCuts cuts;         // streamed; else n_four units in all
+    int n_units;           // of nc cells; streamed: each is taken in quarters
     int* counter;          // streamed
 };
 
@@ -291,8 +291,8 @@ __global__ void __launch_bounds__(kOuterWarps * 32, 1)
     // not streamed: what is left of this CTA's stretch, from row s_from.y of unit s_from.x to row s_to.y of unit s_to.x
     __shared__ int2 s_from, s_to;
     if (!ss.ready) {
-        const int2 from = stretch_cut<W * 32>(op, sc.cuts.n_four, blockIdx.x),
-                   to = stretch_cut<W * 32>(op, sc.cuts.n_four, blockIdx.x + 1);
+        const int2 from = stretch_cut<W * 32>(op.item_cum, op.n_items, sc.n_units, blockIdx.x),
+                   to = stretch_cut<W * 32>(op.item_cum, op.n_items, sc.n_units, blockIdx.x + 1);
         if (tid == 0) {
             s_from = from;
             s_to = to;
@@ -304,9 +304,9 @@ __global__ void __launch_bounds__(kOuterWarps * 32, 1)
         if (ss.ready) {
             if (tid == 0) s_unit = atomicAdd(sc.counter, 1);
             __syncthreads();
-            if (s_unit >= sc.cuts.n_units) break;
-            int bin;
-            unit_of(sc.cuts, s_unit, ht, bin);
+            if (s_unit >= 4 * sc.n_units) break;
+            ht = s_unit / 4;
+            const int bin = 1 + s_unit % 4;
             b0 = sc.bin_begin[bin];
             nb = sc.bin_begin[bin + 1] - b0;
         } else {
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kOuterWarps * 32, 1)
         }
         if (tid == 0 && ss.done) {
             const int h0 = chunk * ss.ht_per_chunk;
-            const int c_ht = min(ss.ht_per_chunk, sc.cuts.n_four - h0);
+            const int c_ht = min(ss.ht_per_chunk, sc.n_units - h0);
             const int c_units = c_ht * 4;  // a streamed launch cuts every half-tile into 4
             if (atomicAdd(ss.done + chunk, 1) == c_units - 1) {
                 __threadfence_system();

@@ -13,14 +13,15 @@
 //
 // What bounds it: shared-memory wavefronts (83 % of peak at K = 5; FP64 pipe 49 %) -- 2 K loads an entry and one
 // wavefront per R_t element -- and, before a row's slices were read ahead and the CTA had more warps than 8,
-// the L2 round trips between slices.  B200, folded, L = 12, K = 5, 2048 cells: 8 warps 1360 us, 16 warps and
-// read-ahead 1045 us, with the last half-tiles in sixteenths 958 us.  Small batches are bound by one row's
+// the L2 round trips between slices.  B200, L = 12, K = 5, 2048 cells, folded: 8 warps 1360 us, 16 warps and
+// read-ahead 1045 us, in stretches of the list of items 926 us.  Stretches against whole half-tiles, quarters and
+// sixteenths (41 items at L = 8 fill 12 warps badly, and every unit stages f): L = 8, 1001 cells, K = 6, plain 246 -> 207
+// us; 4096 cells, K = 4, plain 436 -> 378 us, J.v 655 -> 593 us.  Small batches are bound by one row's
 // slices in sequence and by launches: L = 4, K = 5, 100 cells, plain: layout passes and whole rows 35.7 us,
 // cell-major with rows in parts 18.0 us.
 //
 // The rest follows tile_kernels.cuh: 16-cell half-tile resident in shared memory, R_t staged per
-// warp with cp.async, persistent CTAs pulling whole half-tiles and then binned half-tiles from a
-// device counter, warps pulling pair items from a shared counter.
+// warp with cp.async, a CTA's stretch of the list of all items, warps pulling pair items from a shared counter.
 #pragma once
 #include <type_traits>
 
@@ -30,13 +31,15 @@
 
 namespace cf {
 
+// Work of one launch: the pair items of all half-tiles, heaviest first, half-tile after half-tile, are one list that the
+// CTAs share out in contiguous stretches of equal work (af_tile_kernel).
 struct PairSched {
-    const int* bin_begin;  // bins over pair items: 0 = all (heaviest first), 1..4, 5..20
-    const int* bin_item;   // item indices
+    const int* order;      // item indices, heaviest first
+    const long long* cum;  // [n_items + 1] their work added up
     const int2* items;     // (qa, qb); qb = -1 for a row without a mirror
-    UnitCuts cuts;
-    int* counter;
-    int share;  // items per unit that the shared part sums have room for (0: none)
+    int n_items, n_ht;
+    int n_buf;  // half-tiles resident at a time
+    int share;  // items that the shared part sums have room for (0: none)
 };
 
 template <int K, typename T = double>
@@ -488,120 +491,122 @@ __device__ __forceinline__ void pair_split_item(const DevOp& op, int2 item, cons
 }
 
 // fT, vT: tiled cells in T (FP64 tiles for the FP64 forms, FP32 tiles for the FP32 form); QT: FP64.
-// CM: fT, vT, QT are the caller's cell-major arrays of n_cells cells (FP64 forms).  sc.share: where a unit has
-// fewer items than warps, the warps take (item, part) pairs, of that many items at a time, and the parts are added from
-// shared memory.
+// CM: fT, vT, QT are the caller's cell-major arrays of n_cells cells (FP64 forms).  sc.share: the last, light items
+// that would leave warps idle are shared out by parts, which are added from shared memory at the end.
 template <int K, int W, bool EXACT, bool JV, bool RG, typename T = double, bool SPLIT = false, bool CM = false>
 __global__ void __launch_bounds__(W * 32, sizeof(T) == 8 && K <= 4 && !RG ? 2 : 1)
     af_pair_kernel(DevOp op, PairSched sc, const T* __restrict__ fT, const T* __restrict__ vT,
                    double* __restrict__ QT, long long n_cells) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* smem = reinterpret_cast<T*>(smem_raw);
-    __shared__ int s_unit, s_next;
+    __shared__ int s_next;
     const int M = op.n_q * K;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    T* fs = smem;
-    T* vs = JV ? smem + (size_t)M * kTileCells : nullptr;
+    const int one = M * kTileCells, tile = (JV ? 2 : 1) * one;  // elements of a resident array, of a half-tile
     constexpr bool TS = sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(K, JV);
     constexpr int WB = RPair<K, T>::SIZE + (TS ? K * 32 : 0);  // a warp's elements
-    T* rb = smem + (size_t)(JV ? 2 : 1) * M * kTileCells + (size_t)warp * WB;
+    T* rb = smem + (size_t)sc.n_buf * tile + (size_t)warp * WB;
+    // part sums [item][part][k1][lane] behind the warps' R buffers
+    double* parts = reinterpret_cast<double*>(smem + (size_t)sc.n_buf * tile + (RG ? 0 : (size_t)W * WB));
     constexpr int PER16 = 16 / (int)sizeof(T);    // elements per 16-byte copy
     constexpr int CPR = kTileCells / PER16;       // 16-byte copies per 16-cell row
-    int staged = -1;
+    const int2 from = stretch_cut<W * 32>(sc.cum, sc.n_items, sc.n_ht, blockIdx.x),
+               to = stretch_cut<W * 32>(sc.cum, sc.n_items, sc.n_ht, blockIdx.x + 1);
+    const int last = to.y > 0 ? to.x : to.x - 1;
 
-    for (;;) {
-        if (tid == 0) s_unit = atomicAdd(sc.counter, 1);
-        __syncthreads();
-        const int u = s_unit;
-        if (u >= sc.cuts.n_units) break;
-        int ht, bin;
-        unit_of(sc.cuts, u, ht, bin);
-        const size_t tile_base = (size_t)(ht >> 1) * M * CF_TILE + (size_t)(ht & 1) * kTileCells;
-        const long long cell0 = (long long)ht * kTileCells;
-        if (ht != staged) {
+    for (int h0 = from.x; h0 <= last; h0 += sc.n_buf) {
+        const int n = min(sc.n_buf, last - h0 + 1);
+        int total = 0;  // items of these half-tiles
+        for (int h = h0; h < h0 + n; ++h) {
+            T* fs = smem + (size_t)(h - h0) * tile;
             if constexpr (CM) {
-                stage_cells<K>(fs, fT, op.n_q, cell0, n_cells, tid, W * 32);
-                if constexpr (JV) stage_cells<K>(vs, vT, op.n_q, cell0, n_cells, tid, W * 32);
+                stage_cells<K>(fs, fT, op.n_q, (long long)h * kTileCells, n_cells, tid, W * 32);
+                if constexpr (JV) stage_cells<K>(fs + one, vT, op.n_q, (long long)h * kTileCells, n_cells, tid, W * 32);
             } else {
-                const T* srcf = fT + tile_base;
+                const size_t base = (size_t)(h >> 1) * M * CF_TILE + (size_t)(h & 1) * kTileCells;
                 for (int i = tid; i < M * CPR; i += W * 32) {
                     const int r = i / CPR, w = (i % CPR) * PER16;
-                    cp_async16(fs + r * kTileCells + w, srcf + (size_t)r * CF_TILE + w);
-                }
-                if constexpr (JV) {
-                    const T* srcv = vT + tile_base;
-                    for (int i = tid; i < M * CPR; i += W * 32) {
-                        const int r = i / CPR, w = (i % CPR) * PER16;
-                        cp_async16(vs + r * kTileCells + w, srcv + (size_t)r * CF_TILE + w);
-                    }
+                    cp_async16(fs + r * kTileCells + w, fT + base + (size_t)r * CF_TILE + w);
+                    if constexpr (JV) cp_async16(fs + one + r * kTileCells + w, vT + base + (size_t)r * CF_TILE + w);
                 }
             }
-            cp_async_commit();
-            cp_async_wait_all();
-            staged = ht;
+            total += (h == to.x ? to.y : sc.n_items) - (h == from.x ? from.y : 0);
         }
+        cp_async_commit();
+        cp_async_wait_all();
         if (tid == 0) s_next = 0;
         __syncthreads();
-        const int b0 = sc.bin_begin[bin], nb = sc.bin_begin[bin + 1] - b0;
-        const bool live = !CM || cell0 + (lane & 15) < n_cells;
-        double* qtc = CM ? QT + (size_t)(live ? cell0 + (lane & 15) : 0) * M : QT + tile_base + (lane & 15);
-        if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT) {
-            if (nb < W && (nb <= sc.share || 4 * sc.share >= W)) {
-                // up to sc.share items at a time, in even groups (fewer than a quarter of the warps would leave warps idle: L = 16,
-                // K = 5, 64 cells 506 against 380 us): part sums [item][part][k1][lane] behind the warps' R buffers
-                double* parts = reinterpret_cast<double*>(smem) + (size_t)(JV ? 2 : 1) * M * kTileCells +
-                                (RG ? 0 : (size_t)W * WB);
-                const int groups = (nb + sc.share - 1) / sc.share, size = (nb + groups - 1) / groups;
-                for (int g0 = 0; g0 < nb; g0 += size) {
-                    const int ng = min(size, nb - g0);
-                    for (;;) {
-                        int i = 0;
-                        if (lane == 0) i = atomicAdd(&s_next, 1);
-                        i = __shfl_sync(0xffffffffu, i, 0);
-                        if (i >= ng * kRowParts) break;
-                        double sum[K];
-                        pair_item<K, EXACT, JV, RG, T, CM, TS>(op, sc.items[sc.bin_item[b0 + g0 + i / kRowParts]], fs, vs,
-                                                           rb, qtc, lane, live, i % kRowParts, sum);
-#pragma unroll
-                        for (int k1 = 0; k1 < K; ++k1) parts[(i * K + k1) * 32 + lane] = sum[k1];
-                    }
-                    __syncthreads();
-                    if (tid == 0) s_next = 0;
-                    for (int i = warp; i < ng; i += W) {
-                        const int2 it = sc.items[sc.bin_item[b0 + g0 + i]];
-                        const int q1 = lane < 16 ? it.x : it.y;
-                        if (q1 < 0 || !live) continue;
-#pragma unroll
-                        for (int k1 = 0; k1 < K; ++k1) {
-                            double* out = qtc + q_off<K, CM>(q1, k1, op.n_q);
-                            double x = *out;
-                            for (int g = 0; g < kRowParts; ++g) x += parts[((i * kRowParts + g) * K + k1) * 32 + lane];
-                            *out = x;
-                        }
-                    }
-                    __syncthreads();
-                }
-                continue;
+        // item i of the list: its half-tile (last first: its items are the heavy ones) and rows
+        auto at = [&](int i, int& h) {
+            h = n - 1;
+            for (;; --h) {
+                const int lo = h0 + h == from.x ? from.y : 0, here = (h0 + h == to.x ? to.y : sc.n_items) - lo;
+                if (i < here) return sc.items[sc.order[lo + i]];
+                i -= here;
             }
-        }
+        };
+        auto place = [&](int h, bool& live) {
+            const int ht = h0 + h;
+            const long long cell = (long long)ht * kTileCells + (lane & 15);
+            live = !CM || cell < n_cells;
+            return CM ? QT + (size_t)(live ? cell : 0) * M
+                      : QT + (size_t)(ht >> 1) * M * CF_TILE + (size_t)(ht & 1) * kTileCells + (lane & 15);
+        };
+        int shared = 0;
+        if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT)
+            shared = min(min(sc.share, total), total % W ? total % W : W / 2);
+        const int whole = total - shared;
         for (;;) {
             int i = 0;
             if (lane == 0) i = atomicAdd(&s_next, 1);
             i = __shfl_sync(0xffffffffu, i, 0);
-            if (i >= nb) break;
-            if constexpr (SPLIT)
-                pair_split_item<K, T>(op, sc.items[sc.bin_item[b0 + i]], fs, rb, qtc, lane);
-            else
-                pair_item<K, EXACT, JV, RG, T, CM, TS>(op, sc.items[sc.bin_item[b0 + i]], fs, vs, rb, qtc, lane, live);
+            if (i >= whole + shared * kRowParts) break;
+            const int g = i - whole;  // < 0: a whole item
+            int h;
+            bool live;
+            const int2 item = at(g < 0 ? i : whole + g / kRowParts, h);
+            double* qtc = place(h, live);
+            const T* fs = smem + (size_t)h * tile;
+            if constexpr (SPLIT) {
+                pair_split_item<K, T>(op, item, fs, rb, qtc, lane);
+            } else if constexpr (sizeof(T) == 8 && !EXACT) {
+                double sum[K];
+                pair_item<K, EXACT, JV, RG, T, CM, TS>(op, item, fs, fs + one, rb, qtc, lane, live,
+                                                       g < 0 ? -1 : g % kRowParts, sum);
+                if (g >= 0) {
+#pragma unroll
+                    for (int k1 = 0; k1 < K; ++k1) parts[(g * K + k1) * 32 + lane] = sum[k1];
+                }
+            } else {
+                pair_item<K, EXACT, JV, RG, T, CM, TS>(op, item, fs, fs + one, rb, qtc, lane, live);
+            }
         }
         __syncthreads();
+        if constexpr (sizeof(T) == 8 && !EXACT && !SPLIT) {
+            for (int g = warp; g < shared; g += W) {
+                int h;
+                bool live;
+                const int2 item = at(whole + g, h);
+                double* qtc = place(h, live);
+                const int q1 = lane < 16 ? item.x : item.y;
+                if (q1 < 0 || !live) continue;
+#pragma unroll
+                for (int k1 = 0; k1 < K; ++k1) {
+                    double* out = qtc + q_off<K, CM>(q1, k1, op.n_q);
+                    double x = *out;
+                    for (int p = 0; p < kRowParts; ++p) x += parts[((g * kRowParts + p) * K + k1) * 32 + lane];
+                    *out = x;
+                }
+            }
+            if (shared > 0) __syncthreads();
+        }
     }
 }
 
 // sums: the warps keep row sums behind their R_t (pair_sums_shared)
 template <int K, typename T = double>
-constexpr size_t pair_smem_bytes(int M, int W, bool jv, bool rg, bool sums = false) {
-    return sizeof(T) * ((size_t)(jv ? 2 : 1) * M * kTileCells +
+constexpr size_t pair_smem_bytes(int M, int W, bool jv, bool rg, bool sums = false, int n_buf = 1) {
+    return sizeof(T) * ((size_t)n_buf * (jv ? 2 : 1) * M * kTileCells +
                         (rg ? 0 : (size_t)W * (RPair<K, T>::SIZE + (sums ? K * 32 : 0))));
 }
 

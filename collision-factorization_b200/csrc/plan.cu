@@ -120,6 +120,7 @@ struct cf_plan {
     std::mutex counter_mu;
     int* d_pbin_begin = nullptr; // bins over pair items (same layout as the q1 bins)
     int* d_pbin_item = nullptr;
+    long long* d_pair_cum = nullptr;  // work of the pair items in list order, added up
     int2* d_pitems = nullptr;    // (qa, qb) rows contracted by the two half-warps; qb = -1: no mirror
     int n_pairs = 0, n_pair_items = 0;
     int n_sms = 0;
@@ -295,6 +296,7 @@ void free_plan_memory(cf_plan* p) {
     cudaFree(p->d_counter);
     cudaFree(p->d_pbin_begin);
     cudaFree(p->d_pbin_item);
+    cudaFree(p->d_pair_cum);
     cudaFree(p->d_pitems);
     cudaFree(p->d_ws);
     cudaFree(p->d_io);
@@ -573,6 +575,13 @@ int build_plan(cf_plan* p, const double* labels, const double* vals, const doubl
     CF_TRY(upload(&p->d_bin_q1, bin_q1, bytes));
     CF_TRY(upload(&p->d_pbin_begin, pbin_begin, bytes));
     CF_TRY(upload(&p->d_pbin_item, pbin_item, bytes));
+    std::vector<long long> pair_cum(1, 0);
+    for (int i : porder) {
+        const int q = pitems[i].x;
+        pair_cum.push_back(pair_cum.back() + (long long)(q1_begin[q + 1] - q1_begin[q] + 1) * K +
+                           slice_e[q1_begin[q + 1]] - slice_e[q1_begin[q]]);
+    }
+    CF_TRY(upload(&p->d_pair_cum, pair_cum, bytes));
     CF_TRY(upload(&p->d_pitems, pitems, bytes));
     CF_CUDA(cudaMalloc((void**)&p->d_counter, kCounterSlots * sizeof(int)));
     bytes += kCounterSlots * sizeof(int);
@@ -629,7 +638,7 @@ int dispatch(const cf_plan* p, int what, bool exact, const double* fT, const dou
     // cells/s at L=10, K=8 on B200, J.v 0.59 against 0.75 ms for 2048 cells at L=8, K=8.
     const bool tile_first = p->parent != nullptr && (what == cf::OP_AF || what == cf::OP_JV) && !exact;
     cf::LaunchArgs a{p->op(), fT, vT, QT, nt, B, st, what, exact, p->path, p->d_bin_begin, p->d_bin_q1,
-                     counter_for(p, st), p->n_sms, p->max_smem, p->d_pbin_begin, p->d_pbin_item, p->d_pitems,
+                     counter_for(p, st), p->n_sms, p->max_smem, p->d_pbin_item, p->d_pitems, p->d_pair_cum, p->n_pair_items,
                      fT32 != nullptr, fT32, tile_first, bf16};
     a.ss = ss;
     a.f_cm = f_cm;

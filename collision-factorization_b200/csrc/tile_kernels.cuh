@@ -32,34 +32,6 @@ struct TileSched {
     int* counter;          // zeroed before the launch
 };
 
-// Units of a persistent launch: whole tiles, then tiles cut into 4 row bins, then the last into 16, so that the
-// CTAs end within a sixteenth of a tile's work of one another.
-struct UnitCuts {
-    int n_whole, n_four;  // tiles taken whole; the end of those cut into 4
-    int n_units;
-};
-__host__ __device__ inline void unit_of(const UnitCuts& c, int u, int& tile, int& bin) {
-    const int fours = (c.n_four - c.n_whole) * 4;
-    if (u < c.n_whole) {
-        tile = u;
-        bin = 0;
-    } else if (u < c.n_whole + fours) {
-        tile = c.n_whole + (u - c.n_whole) / 4;
-        bin = 1 + (u - c.n_whole) % 4;
-    } else {
-        tile = c.n_four + (u - c.n_whole - fours) / 16;
-        bin = 5 + (u - c.n_whole - fours) % 16;
-    }
-}
-// Up to a whole tile per CTA in quarters; with `fine` (a sixteenth still occupies a CTA's warps) an eighth of a tile
-// per CTA in sixteenths after them; everything in sixteenths where quarters would not go round once.
-inline UnitCuts cut_units(int64_t n_tiles, int64_t ctas, bool fine) {
-    const int64_t n16 = n_tiles * 4 < ctas ? n_tiles : !fine ? 0 : (n_tiles < ctas / 8 ? n_tiles : ctas / 8);
-    const int64_t n4 = n_tiles - n16 < ctas ? n_tiles - n16 : ctas;
-    const int64_t n_whole = n_tiles - n16 - n4;
-    return {(int)n_whole, (int)(n_whole + n4), (int)(n_whole + n4 * 4 + n16 * 16)};
-}
-
 __host__ __device__ constexpr int bin_base(int split) { return split == 4 ? 1 : 5; }
 
 template <int K>
@@ -68,18 +40,17 @@ struct RBuf {
     static constexpr int SIZE = K * SL;
 };
 
-// The place in the list of all units' rows (item_q1, unit after unit) that is nearest to i / gridDim.x of its work, as
-// (unit, row).  All T threads of the CTA call it.
+// A list of n rows per unit, with the work of rows 0 .. i - 1 in cum[i], unit after unit: the place nearest to
+// i / gridDim.x of its work, as (unit, row).  All T threads of the CTA call it.
 template <int T>
-__device__ __forceinline__ int2 stretch_cut(const DevOp& op, int n_units, int i) {
-    const int n = op.n_items;
-    const long long total = op.item_cum[n], at = total * n_units / gridDim.x * i + total * n_units % gridDim.x * i / gridDim.x;
+__device__ __forceinline__ int2 stretch_cut(const long long* cum, int n, int n_units, int i) {
+    const long long total = cum[n], at = total * n_units / gridDim.x * i + total * n_units % gridDim.x * i / gridDim.x;
     const int u = (int)(at / total);
     const long long rem = at - u * total;
     int r = 0;
     for (int b = 0; b < n; b += T) {
         const int j = b + (int)threadIdx.x;
-        r += __syncthreads_count(j < n && op.item_cum[min(j, n - 1)] + op.item_cum[min(j, n - 1) + 1] <= 2 * rem);
+        r += __syncthreads_count(j < n && cum[min(j, n - 1)] + cum[min(j, n - 1) + 1] <= 2 * rem);
     }
     return r == n ? make_int2(u + 1, 0) : make_int2(u, r);
 }
@@ -337,7 +308,8 @@ __global__ void __launch_bounds__(W * 32, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int one = M * kTileCells, tile = (JV ? 2 : 1) * one;  // elements of a resident array, of a half-tile
     double* rb = smem + (size_t)n_buf * tile + (size_t)warp * RBuf<K>::SIZE;
-    const int2 from = stretch_cut<W * 32>(op, n_ht, blockIdx.x), to = stretch_cut<W * 32>(op, n_ht, blockIdx.x + 1);
+    const int2 from = stretch_cut<W * 32>(op.item_cum, op.n_items, n_ht, blockIdx.x),
+               to = stretch_cut<W * 32>(op.item_cum, op.n_items, n_ht, blockIdx.x + 1);
     const int last = to.y > 0 ? to.x : to.x - 1;
 
     for (int h0 = from.x; h0 <= last; h0 += n_buf) {

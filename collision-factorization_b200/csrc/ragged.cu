@@ -61,7 +61,7 @@ struct Bucket {
 
 struct Unit {
     int bucket, ht, bin;
-    int chunk;  // the streamed host call's upload chunk holding the half-tile (0 elsewhere)
+    int chunk;  // streamed host call: the upload chunk holding the half-tile; resident cell-major step: half-tiles from ht on
 };
 
 // TILE = false: the pair routine (8 warps, one mirrored row pair per warp, whole Phi per lane);
@@ -172,8 +172,12 @@ struct RaggedSync {
 // into the chunk's mapped host word; the host then queues that chunk's download.
 //
 // Resident (rs.ready null; the device steps): the same routine on the callers' cell-major arrays in
-// `ptrs`, with the handle's own work table, no waits and no chunk words -- the whole step in one
-// launch, without layout passes.
+// `ptrs`, no waits and no chunk words -- the whole step in one launch, without layout passes.  Its table
+// (`groups`) gives the warps several half-tiles at a time where one has few rows, heaviest rows first
+// (a half-tile at L = 4 has 25 rows for 16 warps), and cuts those that would outlast a CTA's share of the work: a whole
+// one at L = 10, K = 8 takes 0.95 ms.  B200, L, K = 4, 4; 6, 6; 8, 6; 10, 8 at 40, 30, 20, 10 % of the cells, against whole
+// half-tiles and quarters of as many as there are CTAs at the end: 600 cells 284 -> 135 us, 2500: 978 -> 278, 6000: 986 ->
+// 523, 10000: 982 -> 814, 16384: 1298 -> 1293.
 __global__ void __launch_bounds__(kTW * 32, 1)
     af_ragged_stream_kernel(const Bucket* __restrict__ buckets, const Unit* __restrict__ units, int n_units,
                             int* __restrict__ counter, RaggedSync rs, CmPtrs ptrs) {
@@ -197,7 +201,7 @@ __global__ void __launch_bounds__(kTW * 32, 1)
         const Unit un = units[u];
         const Bucket& bk = s_bk;
         const int M = bk.M, NQ = bk.op.n_q, K = bk.K;
-        const int chunk = un.chunk;
+        const int chunk = un.chunk, n_h = rs.ready ? 1 : un.chunk;
         const long long cell0 = (long long)un.ht * cf::kTileCells;
         const double* fb = rs.ready ? bk.f_cm : ptrs.f[un.bucket];
         double* qb = rs.ready ? bk.q_cm : ptrs.q[un.bucket];
@@ -215,15 +219,17 @@ __global__ void __launch_bounds__(kTW * 32, 1)
                 }
             }
             __syncthreads();
-            // element j = q + N_Q k of cell c goes to row q K + k of the tile
-            for (int i = tid; i < M * cf::kTileCells; i += W * 32) {
-                const int c = i & 15, j = i >> 4;
-                const int r = (j % NQ) * K + j / NQ;
-                if (cell0 + c < bk.cells)
-                    cf::cp_async8(fs + r * cf::kTileCells + c, fb + (size_t)(cell0 + c) * M + j);
-                else
-                    fs[r * cf::kTileCells + c] = 0.0;
-            }
+            // element j = q + N_Q k of cell c goes to row q K + k of its half-tile
+            for (int h = 0; h < n_h; ++h)
+                for (int i = tid; i < M * cf::kTileCells; i += W * 32) {
+                    const int c = i & 15, j = i >> 4;
+                    const int r = h * M + (j % NQ) * K + j / NQ;
+                    const long long cell = cell0 + h * cf::kTileCells + c;
+                    if (cell < bk.cells)
+                        cf::cp_async8(fs + r * cf::kTileCells + c, fb + (size_t)cell * M + j);
+                    else
+                        fs[r * cf::kTileCells + c] = 0.0;
+                }
             cf::cp_async_commit();
             cf::cp_async_wait_all();
             staged_b = un.bucket;
@@ -232,20 +238,21 @@ __global__ void __launch_bounds__(kTW * 32, 1)
         if (tid == 0) s_next = 0;
         __syncthreads();
         const int b0 = bk.bin_begin[un.bin], nb = bk.bin_begin[un.bin + 1] - b0;
-        const long long cell = cell0 + (lane & 15);
-        const bool live = cell < bk.cells;
-        double* qc = qb + (size_t)(live ? cell : 0) * M;
         for (;;) {
             int i = 0;
             if (lane == 0) i = atomicAdd(&s_next, 1);
             i = __shfl_sync(0xffffffffu, i, 0);
-            if (i >= nb) break;
-            const int q1 = bk.bin_q1[b0 + i];
+            if (i >= nb * n_h) break;
+            const int q1 = bk.bin_q1[b0 + i / n_h], h = i % n_h;
+            const long long cell = cell0 + h * cf::kTileCells + (lane & 15);
+            const bool live = cell < bk.cells;
+            double* qc = qb + (size_t)(live ? cell : 0) * M;
+            const double* ft = fs + (size_t)h * M * cf::kTileCells;
             switch (K) {
-                case 2: cf::tile_q1<2, false, false, true>(bk.op, q1, fs, nullptr, rb, qc, lane, live); break;
-                case 4: cf::tile_q1<4, false, false, true>(bk.op, q1, fs, nullptr, rb, qc, lane, live); break;
-                case 6: cf::tile_q1<6, false, false, true>(bk.op, q1, fs, nullptr, rb, qc, lane, live); break;
-                case 8: cf::tile_q1<8, false, false, true>(bk.op, q1, fs, nullptr, rb, qc, lane, live); break;
+                case 2: cf::tile_q1<2, false, false, true>(bk.op, q1, ft, nullptr, rb, qc, lane, live); break;
+                case 4: cf::tile_q1<4, false, false, true>(bk.op, q1, ft, nullptr, rb, qc, lane, live); break;
+                case 6: cf::tile_q1<6, false, false, true>(bk.op, q1, ft, nullptr, rb, qc, lane, live); break;
+                case 8: cf::tile_q1<8, false, false, true>(bk.op, q1, ft, nullptr, rb, qc, lane, live); break;
                 default: break;
             }
         }
@@ -288,6 +295,8 @@ struct cf_ragged {
     double* d_tiles = nullptr;  // per bucket: tiled f, tiled Q
     std::vector<size_t> tile_off;
     int n_units = 0, ctas = 0;
+    Unit* d_groups = nullptr;  // the resident cell-major step's table
+    int n_groups = 0;
     size_t smem = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
@@ -357,6 +366,7 @@ void free_ragged(cf_ragged* r) {
     if (r->graph) cudaGraphDestroy(r->graph);
     cudaFree(r->d_buckets);
     cudaFree(r->d_units);
+    cudaFree(r->d_groups);
     cudaFree(r->d_counter);
     cudaFree(r->d_tiles);
     cudaFree(r->d_io);
@@ -399,8 +409,8 @@ int enqueue_contract(cf_ragged* r, cudaStream_t s, bool count = true) {
 int enqueue_resident_cm(cf_ragged* r, cudaStream_t s, bool count) {
     RCHECK(cudaMemsetAsync(r->d_counter, 0, sizeof(int), s));
     const RaggedSync none{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0};
-    const unsigned grid = (unsigned)std::min(r->n_units, r->ctas);
-    af_ragged_stream_kernel<<<grid, kTW * 32, r->smem, s>>>(r->d_buckets, r->d_units, r->n_units, r->d_counter,
+    const unsigned grid = (unsigned)std::min(r->n_groups, r->ctas);
+    af_ragged_stream_kernel<<<grid, kTW * 32, r->smem, s>>>(r->d_buckets, r->d_groups, r->n_groups, r->d_counter,
                                                             none, r->last_ptrs);
     RCHECK(cudaGetLastError());
     if (count) cf_add_launches(1);
@@ -819,9 +829,35 @@ int cf_ragged_create(cf_ragged** out, cf_plan* const* plans, const int64_t* cell
             }
         }
         r->cell_major = cm;
+        std::vector<Unit> groups;
+        if (cm) {
+            // A CTA's share of the work decides: a half-tile of more than 0.8 of it is taken in tail_split parts, or
+            // where a quarter is still more than two shares in 16 (some 8 rows for 16 warps, but a heavy row alone is half a
+            // quarter's time), and light ones together, as many as give 6 rows a
+            // warp, fit where the largest bucket's one fits and are at most 0.03 of a share.
+            auto cost = [&](int b) { return r->cost[b] * (1.0 + 25.0 / (r->K[b] * r->K[b])); };  // FLOPs, and more per FLOP at small K
+            double share = 0.0;
+            for (const auto& h : hts) share += cost(h.first) / r->ctas;
+            for (size_t i = 0; i < n_ht;) {
+                const int b = hts[i].first, rows = std::max(1, hb[b].op.n_items);
+                int n = 1;
+                if (tail_split > 0 && cost(b) > 0.8 * share) {
+                    const int parts = cost(b) > 8.0 * share ? 16 : tail_split;
+                    for (int k = 0; k < parts; ++k) groups.push_back({b, hts[i].second, (parts == 4 ? 1 : 5) + k, 1});
+                } else {
+                    n = (int)std::min<size_t>(max_M / hb[b].M, (6 * kTW + rows - 1) / rows);
+                    n = std::max(1, (int)std::min((double)n, 0.03 * share / cost(b)));
+                    while (n > 1 && (i + n > n_ht || hts[i + n - 1].first != b)) --n;
+                    groups.push_back({b, hts[i].second, 0, n});
+                }
+                i += n;
+            }
+            r->n_groups = (int)groups.size();
+        }
         e = cudaMalloc(&r->d_tiles, std::max<size_t>(tiles_total, 1) * sizeof(double));
         if (e == cudaSuccess) e = cudaMalloc(&r->d_buckets, n_buckets * sizeof(Bucket));
         if (e == cudaSuccess) e = cudaMalloc(&r->d_units, std::max<size_t>(units.size(), 1) * sizeof(Unit));
+        if (e == cudaSuccess) e = cudaMalloc(&r->d_groups, std::max<size_t>(groups.size(), 1) * sizeof(Unit));
         if (e == cudaSuccess) e = cudaMalloc(&r->d_counter, sizeof(int));
         if (e != cudaSuccess) {
             cf_set_last_error(cudaGetErrorString(e));
@@ -837,6 +873,8 @@ int cf_ragged_create(cf_ragged** out, cf_plan* const* plans, const int64_t* cell
         e = cudaMemcpy(r->d_buckets, hb.data(), n_buckets * sizeof(Bucket), cudaMemcpyHostToDevice);
         if (e == cudaSuccess && !units.empty())
             e = cudaMemcpy(r->d_units, units.data(), units.size() * sizeof(Unit), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && !groups.empty())
+            e = cudaMemcpy(r->d_groups, groups.data(), groups.size() * sizeof(Unit), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             cf_set_last_error(cudaGetErrorString(e));
             st = CF_ECUDA;

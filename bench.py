@@ -69,9 +69,9 @@ NCU_TRAFFIC = {
     ("ragged_hs_b16384", "ragged_tile_0", "af_sym"): (86.450176e6 + 4.645632e6,
                                                      "ncu dram__bytes_read.sum + dram__bytes_write.sum, "
                                                      "profiles/af_ragged_kernel_tile_hs_b16384.md"),
-    ("hs_l10_k8_b4096", "tile_cell_major", "af_sym"): (64.777728e6 + 2.003456e6,
-                                                       "ncu dram__bytes_read.sum + dram__bytes_write.sum, "
-                                                       "profiles/af_tile_stream_kernel_folded_hs_l10_k8_b4096.md"),
+    ("hs_l10_k8_b4096", "outer", "af_sym"): (65.231104e6 + 2.833664e6,
+                                             "ncu dram__bytes_read.sum + dram__bytes_write.sum, "
+                                             "profiles/af_outer_kernel_folded_hs_l10_k8_b4096.md"),
     ("hs_l16_k12_b1024", "lblock", "af_sym"): (74.657024e6 + 9.41312e6,
                                                "ncu dram__bytes_read.sum + dram__bytes_write.sum of the l-block kernel "
                                                "launch (the pack pass before it not counted), "
@@ -540,12 +540,15 @@ def run_ours(args):
         last_path = _lib.PATH_NAMES[op.info()["last_path"]]
         if chosen == "af_sym" and sym_single:
             last_path = "tile_cell_major"
+        if K in (7, 8) and last_path in ("tile", "tile_cell_major") and args.path in (None, "auto"):
+            last_path = "outer"
     traffic = NCU_TRAFFIC.get((args.workload, last_path, chosen))
     kern_name = {"pair": "af_pair_kernel (persistent, tile-resident, mirrored row pairs)",
                  "pair_split": "af_pair_kernel, split variant (both mirrored rows per lane, k3 halves)",
                  "pair_l1": "af_pair_kernel (R_t through L1)", "tile": "af_tile_kernel (persistent, tile-resident)",
-                 "tile_cell_major": "af_tile_stream_kernel, resident (the tile kernel on the cell-major arrays, "
-                                    "no layout passes; the whole device step)",
+                 "tile_cell_major": "af_tile_kernel on the cell-major arrays (no layout passes; the whole device step)",
+                 "outer": "af_outer_kernel (Phi on the FP64 tensor cores, four runs of equal q2 per mma.sync m8n8k4; on the "
+                          "cell-major arrays; the whole device step)",
                  "gather": "af_kernel (gathers through L1/L2)",
                  "tile_mma": "af_mma_kernel (tile-resident, K^3 step on the FP64 MMA)",
                  "split_i8": "af_split_kernel (Phi in FP64 on the folded operator, K^3 step on the int8 tensor cores "

@@ -809,8 +809,8 @@ __global__ void __launch_bounds__(W * 32, 1) af_band64_kernel(SplitArgs a) {
 // At L = 16, K = 12, 1024 cells, against one entry at a time through shuffles: FP64 6.90 -> 6.08 ms,
 // FP32 (with the packed multiply-add) 4.37 -> 3.33 ms, both with the same bits.  What bounds them now is
 // shared-memory bandwidth: an item (14 runs on average) reads 14 x 40 + 144 wavefronts in FP64 (f, the
-// records; the R_t fragments), 71 % of the time at one per clock, beside 582 clocks of the FP64 pipe; in
-// FP32 14 x 26 + 460, 76 %.
+// records; the R_t fragments), 63 % of peak, beside the FP64 datapath (DFMA 34 % and DMMA 30 %); in
+// FP32 14 x 26 + 460, 82 % of peak.
 
 // f cell-major [B][K][N_Q] -> packed [cg][q][k / 2][C][k % 2], or with CELLROWS [cg][q][C][k] (zero past the
 // end of the batch).  One CTA per

@@ -119,7 +119,9 @@ int cf_radial_first(double* Q, const double* f, const double* labels, const doub
  * automatic kernel order; either fast form with kernel path 2) are streamed: one launch over the
  * whole batch starts as soon as the first chunk of cells is on the device and hands each chunk back
  * as soon as it is final, with the same result bits as the device entry points.  Other forms cut
- * the batch into chunks that go up, are contracted and come back on three streams.  Up to 8 cells
+ * the batch into chunks that go up, are contracted and come back on three streams.  Pageable arrays go
+ * through pinned memory of the plan (at most 128 MB, taken once a plan has seen a few such calls) that
+ * several threads copy into and out of.  Up to 8 cells
  * (one f per call, as the reference's MEX is called), the fast forms CF_FORM_AF, CF_FORM_AF_SYM and
  * CF_FORM_RF (K <= 8 for RF) are one launch of the few-cell kernel, with f and Q_in passed in the
  * launch's parameter block when they fit (2 B N_Q K <= 3968 doubles); cf_angular_first and
@@ -189,10 +191,11 @@ int cf_q_tiled(cf_plan* plan, double* q_tiled, const double* f_tiled, int64_t b,
 int cf_jv_tiled(cf_plan* plan, double* out_tiled, const double* f_tiled, const double* v_tiled, int64_t b,
                 int32_t exact, void* stream);
 
-/* Kernel family of a plan's angular-first and Jacobian contractions: 0 = automatic (the first of
- * pair, tile, gather that fits; tile before pair for the fast Q form of the folded operator, whose
- * lighter Phi step favours the tile kernel's higher occupancy; the l-block kernel for the fast Q
- * forms, plain and folded, at K = 12), 1 = the gather kernel (warp per row and 32-cell tile,
+/* Kernel family of a plan's angular-first and Jacobian contractions: 0 = automatic (for the fast
+ * forms at K = 7 and 8 the outer-product kernels, Phi on the FP64 tensor cores, reported as 2 or 8;
+ * else the first of pair, tile, gather that fits; tile before pair for the fast forms of the folded
+ * operator, whose lighter Phi step favours the tile kernel's higher occupancy; the l-block kernel for
+ * the fast Q forms, plain and folded, at K = 12), 1 = the gather kernel (warp per row and 32-cell tile,
  * f read through L1/L2), 2 = the tile-resident kernel (16 cells in shared memory, Phi split over
  * two lanes per cell), 3 = the pair kernel (16 cells in shared memory, the mirrored rows (l,+m) and
  * (l,-m) on the two half-warps), 4 = the pair kernel reading R through L1 instead of shared
@@ -256,7 +259,9 @@ int cf_plan_lblock_selftest(cf_plan* plan, double wait_seconds);
  * its own plan's kernels in the same step.  family picks the routine of the fused launch: 0 the
  * pair routine (8 warps per CTA), 1 the tile routine (16 warps per CTA; buckets of odd K then run
  * on their own).  tail_split (0, 4 or 16) is how many bins each of the last half-tiles of the fused
- * work table is cut into, so that the launch ends evenly.
+ * work table is cut into, so that the launch ends evenly (0: none is cut); the one launch on the
+ * cell-major arrays cuts the half-tiles that would outlast a CTA's share of the step's work, into
+ * that many bins or 16.
  * cf_ragged_q enqueues pack, fused launch, the separate buckets and unpack on the stream (when every
  * non-empty bucket is fused on the tile routine: one launch on the cell-major arrays instead);
  * cf_ragged_graph_launch records that sequence into a CUDA graph on first use (per set of buffers)

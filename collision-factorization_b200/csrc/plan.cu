@@ -752,17 +752,40 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
     if (B < 0) return fail(CF_ESHAPE, "B = %lld is negative", (long long)B);
     if (B == 0 || p->n_g == 0) return CF_OK;
     if (!q_dev || !f_dev || (what == 2 && !v_dev)) return fail(CF_EINVAL, "null device buffer");
+    // The routes that read f (and v) and add to Q in the caller's arrays have CTAs that read cells whose Q another CTA
+    // has already added to.  Where Q shares memory with f or v they read copies of the inputs, made in the workspace
+    // (which these routes leave unused); the others (layout passes, packed f) copy their inputs before they write.
+    const size_t n_in = (size_t)B * p->n_q * p->k;
+    auto shares = [&](const double* x) { return (uintptr_t)x < (uintptr_t)(q_dev + n_in) && (uintptr_t)q_dev < (uintptr_t)(x + n_in); };
+    const bool shared = shares(f_dev) || (what == 2 && shares(v_dev));
+    const double *f_in = f_dev, *v_in = v_dev;
+    auto own_inputs = [&]() -> int {
+        if (!shared || f_in != f_dev) return CF_OK;
+        const size_t slot = tiled_bytes(p, B), have = ws ? ws_bytes : 0;
+        if (have < slot * (what == 2 ? 2 : 1))
+            return fail(CF_EINVAL, "Q overlaps an input: a workspace of %zu bytes does not hold the inputs' copies", have);
+        CF_CUDA(cudaMemcpyAsync(ws, f_dev, n_in * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        f_in = (const double*)ws;
+        if (what == 2) {
+            v_in = (const double*)((char*)ws + slot);
+            CF_CUDA(cudaMemcpyAsync((char*)ws + slot, v_dev, n_in * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        }
+        return CF_OK;
+    };
     if (f32 == 3) {
         if (what != 0) return fail(CF_EUNSUPPORTED, "the split form computes Q only");
-        return run_split(p, q_dev, f_dev, B, st);
+        CF_TRY(own_inputs());
+        return run_split(p, q_dev, f_in, B, st);
     }
     if (f32 == 4) {
         if (what != 0) return fail(CF_EUNSUPPORTED, "the radial-first dense form computes Q only");
         return run_rfdense(p, q_dev, f_dev, B, st);
     }
-    {
-        const int r = run_few(p, what, exact, q_dev, f_dev, B, st, sym, f32);
+    if (B <= kFewCells && what != 2 && f32 == 0) {
+        CF_TRY(own_inputs());
+        const int r = run_few(p, what, exact, q_dev, f_in, B, st, sym, f32);
         if (r != kNoFew) return r;
+        f_in = f_dev;  // the routes below that want the copy make it again: a layout pass may come first
     }
     // The exact angular-first form and the exact J.v above K = 8, where the batch kernels' per-lane
     // K x K Phi does not fit in registers: the row kernel of the few-cell route (one CTA per (q1, pair of
@@ -771,8 +794,9 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
         if (B > 65535)
             return fail(CF_ESHAPE, "the exact forms above K = 8 take at most 65535 cells per call (B = %lld)",
                         (long long)B);
-        const int r = dispatch(p, what, true, nullptr, nullptr, nullptr, B, st, nullptr, false, nullptr, f_dev, q_dev,
-                               true, nullptr, nullptr, nullptr, true, what == 2 ? v_dev : nullptr);
+        CF_TRY(own_inputs());
+        const int r = dispatch(p, what, true, nullptr, nullptr, nullptr, B, st, nullptr, false, nullptr, f_in, q_dev,
+                               true, nullptr, nullptr, nullptr, true, what == 2 ? v_in : nullptr);
         if (r != kNoFew) return r;
     }
     const size_t tb = tiled_bytes(p, B);
@@ -785,9 +809,10 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
         cf_plan* target = p;
         if (sym) CF_TRY(get_sym(p, &target));
         if (!streamable(p, target, what, exact, f32)) CF_TRY(check_tiles(B));
+        CF_TRY(own_inputs());
         const StreamSync resident{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, 0};
-        return dispatch(target, what, false, nullptr, nullptr, nullptr, B, st, nullptr, false, &resident, f_dev, q_dev,
-                        false, nullptr, nullptr, nullptr, false, what == 2 ? v_dev : nullptr);
+        return dispatch(target, what, false, nullptr, nullptr, nullptr, B, st, nullptr, false, &resident, f_in, q_dev,
+                        false, nullptr, nullptr, nullptr, false, what == 2 ? v_in : nullptr);
     }
     double* fT = (double*)ws;
     double* QT = (double*)((char*)ws + tb);
@@ -797,8 +822,10 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
         cf_plan* target = p;
         if (sym) CF_TRY(get_sym(p, &target));
         if (!exact && f32 == 0) {
-            int r = run_band64(target, q_dev, f_dev, B, st);
+            if (target->path == cf::PATH_BAND) CF_TRY(own_inputs());
+            int r = run_band64(target, q_dev, f_in, B, st);
             if (r != kNoFew) return r;
+            f_in = f_dev;
             r = run_lblock(target, q_dev, f_dev, B, ws, ws_bytes, st, false);
             if (r != kNoFew) return r;
         }
@@ -807,12 +834,14 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
             if (r != kNoFew) return r;
         }
         if (!exact && f32 == 2) {
-            const int r = run_bf16_band(target, q_dev, f_dev, B, st);
+            CF_TRY(own_inputs());
+            const int r = run_bf16_band(target, q_dev, f_in, B, st);
             if (r != kNoFew) return r;
         }
         if (streamable(p, target, what, exact, f32)) {
+            CF_TRY(own_inputs());
             const StreamSync resident{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, 0};
-            return dispatch(target, 0, false, nullptr, nullptr, nullptr, B, st, nullptr, false, &resident, f_dev,
+            return dispatch(target, 0, false, nullptr, nullptr, nullptr, B, st, nullptr, false, &resident, f_in,
                             q_dev);
         }
     }
@@ -825,8 +854,9 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
         cf_plan* target = p;
         if (sym) CF_TRY(get_sym(p, &target));
         CF_TRY(check_tiles(B));
-        return dispatch(target, what, false, nullptr, nullptr, nullptr, B, st, nullptr, false, nullptr, f_dev, q_dev,
-                        false, nullptr, nullptr, nullptr, false, what == 2 ? v_dev : nullptr, true);
+        CF_TRY(own_inputs());
+        return dispatch(target, what, false, nullptr, nullptr, nullptr, B, st, nullptr, false, nullptr, f_in, q_dev,
+                        false, nullptr, nullptr, nullptr, false, what == 2 ? v_in : nullptr, true);
     }
     float* vT32 = (f32 && what == 2) ? reinterpret_cast<float*>(vT) : nullptr;  // FP32 J.v: v's FP32 tiles
     if (f32)

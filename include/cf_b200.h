@@ -165,7 +165,10 @@ int cf_plan_get_info(const cf_plan* plan, cf_plan_info* info);
  * them allocation-free; the other calls allocate it inside the plan on first use. */
 int cf_plan_workspace_size(const cf_plan* plan, int64_t b, int32_t jacobian, size_t* bytes);
 
-/* Q_dev += Q(f_dev) for B cells. */
+/* Q_dev += Q(f_dev) for B cells.  Q_dev may be f_dev itself or overlap it, and out_dev below f_dev or v_dev:
+ * the inputs are read as they were before the call (from copies in the workspace, where the kernel would
+ * otherwise read cells that it has already added to).  The tiled entries and the ragged step need arrays
+ * of their own for Q. */
 int cf_q_device(cf_plan* plan, double* q_dev, const double* f_dev, int64_t b, int32_t form,
                 void* stream);
 int cf_q_device_ws(cf_plan* plan, double* q_dev, const double* f_dev, int64_t b, int32_t form,

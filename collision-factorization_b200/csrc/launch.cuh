@@ -114,6 +114,10 @@ constexpr bool outer_takes(int K, bool folded, bool jv, int64_t n_cells, int n_s
 // with rows of NQP doubles per cell fixed at compile time (one of two widths, 4 modulo 8, so that the 8 lanes
 // of a 128-bit load phase, 2 k x 4 q distinct modulo 4, hit distinct banks) and an odd pair stride.
 constexpr int outer_nqp(int width) { return width == 0 ? 132 : 268; }  // L <= 10, L <= 15
+// Rows of zeros behind the last q (at least one), which a chunk's empty places read: four where there is room, one
+// for each residue modulo 4.
+constexpr int kOuterZeros = 4;
+constexpr int outer_zeros(int n_q, int nqp) { return nqp - n_q < kOuterZeros ? nqp - n_q : kOuterZeros; }
 constexpr int outer_pair(int K, int nqp) { return K * nqp + 1; }       // 16-byte elements per pair of cells
 constexpr int kOuterCells = 4;   // cells per warp: 128 registers a lane hold acc and Phi, 16 warps fit
 constexpr int kOuterWarps = 16;
@@ -135,8 +139,8 @@ struct OuterFit {
     int width, nc;
 };
 constexpr OuterFit outer_fit(int n_q, int K, bool jv, size_t max_smem) {
-    const int width = n_q <= outer_nqp(0) ? 0 : 1;
-    if (n_q > outer_nqp(width)) return {0, 0};
+    const int width = n_q < outer_nqp(0) ? 0 : 1;
+    if (n_q >= outer_nqp(width)) return {0, 0};
     for (int nc = 16; nc >= 8; nc -= 8)
         if (outer_smem_bytes(n_q, K, outer_nqp(width), nc, jv) + 256 <= max_smem) return {width, nc};
     return {0, 0};

@@ -15,8 +15,9 @@
 //
 // Cells lie in shared memory in pairs, [pair][k][q][2], with the q rows padded to 4 modulo 8 pairs: the 8 lanes of
 // a 128-bit phase (2 k x 4 runs) hit distinct banks when the runs' q are distinct modulo 4, which the host
-// arranges when it packs runs into chunks (plan.cu, build_outer).  Empty slots of a chunk repeat a run of
-// the chunk with G = 0, so they read nothing the slice does not read and add nothing.
+// arranges when it packs runs into chunks (plan.cu, build_outer).  Empty slots of a chunk, and the second q3 of
+// a run of one in a chunk of two, have G = 0 and read rows of zeros behind the last q: a product of zeros adds nothing,
+// also where the slice's own f is infinite.
 //
 // What bounds it: shared-memory wavefronts (72 % of peak at L = 10, K = 8: 17 a cell and slice for the Phi operands,
 // 8 for R_t, 8 for chunks, heads and copies), with the FP64 pipe at 50 %.  Four cells a warp (128 registers,
@@ -287,6 +288,13 @@ __global__ void __launch_bounds__(kOuterWarps * 32, 1)
     const int team_warps = g.nc / kOuterCells, team = warp / team_warps, w_in_team = warp - team * team_warps;
     OuterTask* tasks = reinterpret_cast<OuterTask*>(rings + 2 * (W / team_warps));
     const size_t mine = (size_t)w_in_team * (kOuterCells / 2) * outer_pair(K, NQP);  // this warp's cells
+    // the rows of zeros, which staging leaves alone
+    const int n_zero = outer_zeros(op.n_q, NQP);
+    for (int i = tid; i < (JV ? 2 : 1) * (g.nc / 2) * K * n_zero; i += W * 32) {
+        const int row = i / n_zero, pair = row / K;
+        reinterpret_cast<double2*>(fs)[(size_t)pair * outer_pair(K, NQP) + row % K * NQP + op.n_q + i % n_zero] =
+            make_double2(0.0, 0.0);
+    }
     int staged = -1;
     // not streamed: what is left of this CTA's stretch, from row s_from.y of unit s_from.x to row s_to.y of unit s_to.x
     __shared__ int2 s_from, s_to;

@@ -338,6 +338,7 @@ int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<
     std::vector<unsigned char> xb;
     xs.reserve(S + S / 8);
     xb.reserve((e_q23.size() / 3 + S) * sizeof(Chunk));
+    const int n_zero = cf::outer_zeros(p->n_q, cf::outer_nqp(cf::outer_fit(p->n_q, p->k, false, p->max_smem).width));
     std::vector<uint64_t> ent;  // q2 << 32 | entry
     std::vector<Run> all, one;
     size_t n_chunks = 0;
@@ -364,6 +365,7 @@ int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<
         const int begin = (int)n_chunks;
         for (size_t i0 = 0; i0 < all.size(); i0 += 4) {
             int used[3][4] = {};  // residues taken in this chunk: q2, q3a, q3b
+            const bool two = i0 < n_two;  // the kernel reads q3b too
             for (size_t i = i0; i < std::min(i0 + 4, all.size()); ++i) {
                 const size_t hi = std::min(i + kLook, i < n_two ? n_two : all.size());  // runs of two stay in front
                 size_t best = i;
@@ -389,15 +391,26 @@ int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<
                 ++used[1][r.qa & 3];
                 ++used[2][r.qb & 3];
             }
+            // the row of zeros in the residue that the fewest others of its kind have
+            auto zero_row = [&](int kind) {
+                int best = 0;
+                for (int z = 1; z < n_zero; ++z)
+                    if (used[kind][(p->n_q + z) & 3] < used[kind][(p->n_q + best) & 3]) best = z;
+                ++used[kind][(p->n_q + best) & 3];
+                return (unsigned short)(16 * (p->n_q + best));
+            };
             Chunk c;
             for (size_t i = 0; i < 4; ++i) {
-                // an empty slot repeats the chunk's first run with G = 0
-                const bool in = i0 + i < all.size();
-                const Run& r = all[in ? i0 + i : i0];
-                // as byte offsets in a row of cell pairs (N_Q <= 268 where the kernels run)
-                c.q[i] = make_ushort4((unsigned short)(16 * r.q2), (unsigned short)(16 * r.qa),
-                                      (unsigned short)(16 * r.qb), 0);
-                c.g[i] = in ? make_double2(r.ga, r.gb) : make_double2(0.0, 0.0);
+                // as byte offsets in a row of cell pairs (N_Q < 268 where the kernels run)
+                if (i0 + i < all.size()) {
+                    const Run& r = all[i0 + i];
+                    c.q[i] = make_ushort4((unsigned short)(16 * r.q2), (unsigned short)(16 * r.qa),
+                                          r.two || !two ? (unsigned short)(16 * r.qb) : zero_row(2), 0);
+                    c.g[i] = make_double2(r.ga, r.gb);
+                } else {
+                    c.q[i] = make_ushort4(zero_row(0), zero_row(1), zero_row(2), 0);
+                    c.g[i] = make_double2(0.0, 0.0);
+                }
             }
             xb.insert(xb.end(), (const unsigned char*)&c, (const unsigned char*)(&c + 1));
             ++n_chunks;

@@ -890,8 +890,9 @@ struct LbMma {
 };
 
 // The Phi step reads run records: up to two entries (q2, q3a, G a), (q2, q3b, G b) of a slice with the
-// same q2 (the selection rules allow two m3 per (m1, m2); a longer run takes several records), a missing
-// second entry as G b = 0 on q3a.  The rows' offsets in the stage are in bytes, so a run costs no index
+// same q2 (the selection rules allow two m3 per (m1, m2); a longer run takes several records), a single
+// entry as two halves (G / 2 + G / 2 on one q3: the same rounding as G alone, and an infinite f stays infinite, which a
+// second product with G = 0 would make NaN).  The rows' offsets in the stage are in bytes, so a run costs no index
 // arithmetic, and both kernels read run i + 1 while they multiply run i.  FP64: 32 bytes {Ga, Gb, off2,
 // off3a, off3b, -}; FP32: 16 bytes {Ga, Gb, off2, off3a / 16 | off3b / 16 << 16}.
 template <typename T>
@@ -1890,7 +1891,8 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
                     for (int z = slice_e[sl]; z < slice_e[sl + 1];) {
                         const uint32_t q2 = e_q23[z] & 0xffffu, q3 = e_q23[z] >> 16;
                         const bool two = z + 1 < slice_e[sl + 1] && (e_q23[z + 1] & 0xffffu) == q2;
-                        add_run(e_g[z], two ? e_g[z + 1] : 0.0, q2 - b2, q3 - b3,
+                        const double g = two ? e_g[z] : 0.5 * e_g[z];
+                        add_run(g, two ? e_g[z + 1] : g, q2 - b2, q3 - b3,
                                 (two ? e_q23[z + 1] >> 16 : q3) - b3);
                         z += two ? 2 : 1;
                     }

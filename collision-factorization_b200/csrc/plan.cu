@@ -734,7 +734,7 @@ int launch_unpack(const cf_plan* p, const double* src, double* dst, int64_t B, c
 // the caller's cell-major arrays (the same per-row operations, so the same bits).  So do the fast
 // FP64 Q forms on at most kFewCells cells, on the few-cell kernel (one launch).
 int get_sym(cf_plan* p, cf_plan** out);
-bool streamable(const cf_plan* p, const cf_plan* target, int what, bool exact, int f32);
+bool tile_resident(const cf_plan* p, const cf_plan* target, int what, bool exact, int f32);
 int run_split(cf_plan* p, double* q_dev, const double* f_dev, int64_t B, cudaStream_t st);
 int run_band64(cf_plan* target, double* q_dev, const double* f_dev, int64_t B, cudaStream_t st);
 int run_lblock(cf_plan* target, double* q_dev, const double* f_dev, int64_t B, void* ws, size_t ws_bytes,
@@ -821,7 +821,7 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
         cf::outer_fit(p->n_q, p->k, what == 2, p->max_smem).nc > 0) {
         cf_plan* target = p;
         if (sym) CF_TRY(get_sym(p, &target));
-        if (!streamable(p, target, what, exact, f32)) CF_TRY(check_tiles(B));
+        if (!tile_resident(p, target, what, exact, f32)) CF_TRY(check_tiles(B));
         CF_TRY(own_inputs());
         const StreamSync resident{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, 0};
         return dispatch(target, what, false, nullptr, nullptr, nullptr, B, st, nullptr, false, &resident, f_in, q_dev,
@@ -851,7 +851,7 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
             const int r = run_bf16_band(target, q_dev, f_in, B, st);
             if (r != kNoFew) return r;
         }
-        if (streamable(p, target, what, exact, f32)) {
+        if (tile_resident(p, target, what, exact, f32)) {
             CF_TRY(own_inputs());
             const StreamSync resident{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, 0};
             return dispatch(target, 0, false, nullptr, nullptr, nullptr, B, st, nullptr, false, &resident, f_in,
@@ -1385,14 +1385,21 @@ bool plan_by_pointers(cf_plan** out, uint64_t* key, const double* labels, const 
     return false;
 }
 
-// Streamed host path: whether the fast angular-first form on `target` runs on the tile kernel (so the
-// streamed kernel reproduces the device path bit for bit) and the tile fits in shared memory.
-bool streamable(const cf_plan* p, const cf_plan* target, int what, bool exact, int f32) {
+// Whether the fast angular-first form on `target` is the tile kernel's on the cell-major arrays (before the
+// outer-product kernel, which takes such forms at K = 8) and its tile fits in shared memory.
+bool tile_resident(const cf_plan* p, const cf_plan* target, int what, bool exact, int f32) {
     if (what != 0 || exact || f32 != 0 || p->k % 2 != 0 || p->k > 8) return false;
     const bool tile = target->parent != nullptr ? (p->path == 0 || p->path == cf::PATH_TILE) : p->path == cf::PATH_TILE;
     if (!tile) return false;
     const size_t smem = sizeof(double) * ((size_t)p->n_q * p->k * 16 + (size_t)16 * p->k * (p->k * p->k + 2));
     return smem + 256 <= p->max_smem;
+}
+
+// Streamed host path: whether a streamed launch runs the device path's kernel, so that it gives the same bits.  The
+// outer-product kernel streams units of 16 cells; where it takes units of 8 (K = 8 above L = 10), host calls are chunked.
+bool streamable(const cf_plan* p, const cf_plan* target, int what, bool exact, int f32) {
+    if (!tile_resident(p, target, what, exact, f32)) return false;
+    return p->path != cf::PATH_AUTO || !cf::outer_for(p->k) || cf::outer_fit(p->n_q, p->k, false, p->max_smem).nc != 8;
 }
 
 int ensure_stream_sync(cf_plan* p) {

@@ -228,7 +228,7 @@ static LaunchResult launch_outer(const LaunchArgs& a) {
 template <int K, int W, bool EXACT, bool JV, bool RG, typename T = double, bool SPLIT = false, bool CM = false>
 static LaunchResult launch_pair(const LaunchArgs& a) {
     const int M = a.op.n_q * K;
-    constexpr bool SUMS = sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(K, JV);
+    constexpr bool SUMS = sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(W, JV);
     size_t smem = pair_smem_bytes<K, T>(M, W, JV, RG, SUMS);
     if (smem + 256 > a.max_smem || a.n_pitems == 0) return {-1, 0, cudaSuccess, PATH_PAIR};
     static_assert(!SPLIT || (!EXACT && !JV && !RG && K % 2 == 0), "the split variant is the fast Q form");
@@ -486,9 +486,12 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
     if (a.pair_cm) {
         if constexpr (K <= 8) {
             if (a.what != OP_RF && !a.exact && !a.f32) {
-                const LaunchResult r =
+                LaunchResult r =
                     a.what == OP_JV ? launch_pair<K, pair_W(K, true), false, true, false, double, false, true>(a)
                                     : launch_pair<K, pair_W(K), false, false, false, double, false, true>(a);
+                if (r.status == -1 && pair_W(K, a.what == OP_JV) > 8)  // fewer copies of R_t
+                    r = a.what == OP_JV ? launch_pair<K, 8, false, true, false, double, false, true>(a)
+                                        : launch_pair<K, 8, false, false, false, double, false, true>(a);
                 if (r.status != -1) return r;
             }
         }
@@ -594,8 +597,9 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
                 else
                     r = a.exact ? launch_pair<K, 8, true, false, false>(a) : launch_pair<K, pair_W(K), false, false, false>(a);
             }
-            if (r.status == -1 && a.path != PATH_PAIR_L1 && jv && !a.exact && pair_W(K, true) > 8)
-                r = launch_pair<K, 8, false, true, false>(a);  // fewer copies of R_t
+            if (r.status == -1 && a.path != PATH_PAIR_L1 && !a.exact && pair_W(K, jv) > 8 &&
+                (a.path != PATH_AUTO || pair_auto(a.op.n_q, K, a.tile_first, jv, a.n_cells, a.max_smem)))  // fewer copies of R_t
+                r = jv ? launch_pair<K, 8, false, true, false>(a) : launch_pair<K, 8, false, false, false>(a);
             if (r.status != -1) return r;
             if (a.path != PATH_AUTO) return {8, 0, cudaSuccess, a.path};
         }

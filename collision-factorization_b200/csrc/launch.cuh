@@ -91,12 +91,24 @@ constexpr int af_P(int K) { return K <= 8 ? 1 : (K <= 12 ? 2 : 4); }
 // lane; K = 6, and J.v at K = 5: 168; else 255, or several CTAs on an SM below K = 5).
 constexpr int pair_W(int K, bool jv = false) { return K == 5 ? (jv ? 12 : 16) : (K == 6 && !jv ? 12 : 8); }
 // Shared memory of a warp: R_t and, where registers are short (the 16- and 12-warp Q forms), the row sums.
-constexpr bool pair_sums_shared(int K, bool jv) { return pair_W(K, jv) > 8 && !jv; }
-constexpr int pair_warp_doubles(int K, bool jv) { return (K * K * K + 1) / 2 * 2 + (pair_sums_shared(K, jv) ? K * 32 : 0); }
-// Whether the FP64 pair kernel's 16-cell tile of f (and v) fits beside its warps' copies of R_t.
-constexpr bool pair_fits(int n_q, int K, bool jv, size_t max_smem) {
-    return K <= 8 && sizeof(double) * ((size_t)(jv ? 2 : 1) * n_q * K * 16 + (size_t)pair_W(K, jv) * pair_warp_doubles(K, jv)) +
-                             256 <= max_smem;
+constexpr bool pair_sums_shared(int W, bool jv) { return W > 8 && !jv; }
+constexpr int pair_warp_doubles(int K, int W, bool jv) { return (K * K * K + 1) / 2 * 2 + (pair_sums_shared(W, jv) ? K * 32 : 0); }
+// The FP64 pair kernel's warps where its 16-cell tile of f (and v) fits beside their copies of R_t: pair_W, or 8 where
+// only these fit (Q at L = 17, K = 5 and at L = 15, K = 6); 0 where neither does.
+constexpr int pair_fit(int n_q, int K, bool jv, size_t max_smem) {
+    if (K > 8) return 0;
+    for (int W : {pair_W(K, jv), 8})
+        if (sizeof(double) * ((size_t)(jv ? 2 : 1) * n_q * K * 16 + (size_t)W * pair_warp_doubles(K, W, jv)) + 256 <= max_smem)
+            return W;
+    return 0;
+}
+// Whether the automatic order takes the pair kernel where it fits.  With 8 warps for want of room the gather kernel (folded,
+// K = 5) and the tile kernel (plain, K = 6) are the faster ones on some batches (B200, us, pair / other): L = 17, K = 5 folded:
+// 100 cells 422 / 529, 300: 923 / 853, 2048: 4859 / 4279 (plain 7850 / 8402); L = 15, K = 6 plain: 20 cells 400 / 292, 100:
+// 493 / 431, 300: 1143 / 1137, 1000: 2984 / 3106.
+constexpr bool pair_auto(int n_q, int K, bool folded, bool jv, int64_t n_cells, size_t max_smem) {
+    if (jv || pair_fit(n_q, K, jv, max_smem) == pair_W(K, jv)) return true;
+    return K % 2 ? !folded || n_cells <= 200 : n_cells > 300;
 }
 constexpr int kTileBufs = 4;  // half-tiles that a CTA of the tile kernel holds at a time, at most
 // K that the outer-product kernels (outer_kernels.cuh) take.

@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(W * 32, sizeof(T) == 8 && K <= 4 && !RG ? 2 : 
     const int M = op.n_q * K;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int one = M * kTileCells, tile = (JV ? 2 : 1) * one;  // elements of a resident array, of a half-tile
-    constexpr bool TS = sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(K, JV);
+    constexpr bool TS = sizeof(T) == 8 && !EXACT && !RG && !SPLIT && pair_sums_shared(W, JV);
     constexpr int WB = RPair<K, T>::SIZE + (TS ? K * 32 : 0);  // a warp's elements
     T* rb = smem + (size_t)sc.n_buf * tile + (size_t)warp * WB;
     // part sums [item][part][k1][lane] behind the warps' R buffers

@@ -862,8 +862,9 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
     // arrays, without the layout passes (three or four launches of 2-5 us each).  A batch within one
     // half-tile keeps the passes.
     if (!exact && f32 == 0 && (what == 0 || what == 2) && B > 16 &&
-        (p->path == cf::PATH_PAIR || (p->path == cf::PATH_AUTO && !(sym && p->k % 2 == 0))) &&
-        cf::pair_fits(p->n_q, p->k, what == 2, p->max_smem)) {
+        (p->path == cf::PATH_PAIR || (p->path == cf::PATH_AUTO && !(sym && p->k % 2 == 0) &&
+                                      cf::pair_auto(p->n_q, p->k, sym, what == 2, B, p->max_smem))) &&
+        cf::pair_fit(p->n_q, p->k, what == 2, p->max_smem) > 0) {
         cf_plan* target = p;
         if (sym) CF_TRY(get_sym(p, &target));
         CF_TRY(check_tiles(B));

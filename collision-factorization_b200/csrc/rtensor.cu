@@ -192,21 +192,23 @@ __device__ __forceinline__ double post_velocity(const Dev& d, const Point& P, in
 // operands of a warp, 8 rows x 4 columns, then fall into distinct banks).
 struct ItemLayout {
     int vs, ld;             // points per side and round; column stride
+    int s_out;              // S in device memory: doubles per CTA (0: in shared memory)
     int parts;              // threads per (velocity, function family): they share out m or l
     size_t y, rv, s, rl, pts, tab, total;  // offsets in doubles
 };
 
 // Gain and loss accumulation of one job's items; writes the items' net vectors and radial values.
+template <bool S_OUT>
 __global__ void __launch_bounds__(kItemThreads)
     k_items(Dev d, ItemLayout lay, int64_t group0, int64_t n_groups, int64_t item0, int64_t n_items_chunk,
-            double* __restrict__ net, double* __restrict__ radv) {
+            double* __restrict__ net, double* __restrict__ radv, double* __restrict__ s_scratch) {
     extern __shared__ __align__(16) double sm[];
     const int NK = d.NK, L = d.L, NR = (L + 1) * NK;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int VS = lay.vs, LD = lay.ld;
     double* Y = sm + lay.y;      // [2][n_slots][LD]: W Y_q of the round's velocities
     double* RV = sm + lay.rv;    // [2][NR][LD]: radial functions of the round's velocities
-    double* S = sm + lay.s;      // [2][n_rows][NK]
+    double* S = S_OUT ? s_scratch + (size_t)blockIdx.x * lay.s_out : sm + lay.s;  // [2][n_rows][NK]
     double* RL = sm + lay.rl;    // [2][NR]: radial functions at vL and vS
     Point* pts = reinterpret_cast<Point*>(sm + lay.pts);
     double* inv = sm + lay.tab;  // [32] 1 / n
@@ -483,13 +485,16 @@ __global__ void __launch_bounds__(256) k_reduce(const double* __restrict__ part,
 __global__ void __launch_bounds__(256) k_transpose(const double* __restrict__ src, int64_t rows, int64_t cols,
                                                    double* __restrict__ dst) {
     __shared__ double t[32][33];
-    const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
+    const int64_t c0 = (int64_t)blockIdx.x * 32;
     const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
-    for (int j = y; j < 32; j += 8)
-        if (r0 + j < rows && c0 + x < cols) t[j][x] = src[(r0 + j) * cols + c0 + x];
-    __syncthreads();
-    for (int j = y; j < 32; j += 8)
-        if (c0 + j < cols && r0 + x < rows) dst[(c0 + j) * rows + r0 + x] = t[x][j];
+    for (int64_t r0 = (int64_t)blockIdx.y * 32; r0 < rows; r0 += (int64_t)gridDim.y * 32) {
+        for (int j = y; j < 32; j += 8)
+            if (r0 + j < rows && c0 + x < cols) t[j][x] = src[(r0 + j) * cols + c0 + x];
+        __syncthreads();
+        for (int j = y; j < 32; j += 8)
+            if (c0 + j < cols && r0 + x < rows) dst[(c0 + j) * rows + r0 + x] = t[x][j];
+        __syncthreads();
+    }
 }
 
 typedef void (*ContractFn)(Dev, const double*, const double*, int64_t, double*);
@@ -654,7 +659,7 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
     char* arena = nullptr;
     Dev d{};
     double *net = nullptr, *radv = nullptr, *dR = nullptr, *part = nullptr, *turn = nullptr;
-    double *dg1 = nullptr, *dg2 = nullptr;
+    double *dg1 = nullptr, *dg2 = nullptr, *s_scratch = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     const int NR = (L + 1) * NK;
     // an item of patch 1 without t nodes adds nothing
@@ -669,6 +674,7 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
     int n_split = 1;
     std::vector<char> small;
     ContractFn contract = contract_for(NK);
+    auto items = k_items<false>;
     d.NK = NK;
     d.NL = NL;
     d.NQ = NQ;
@@ -692,10 +698,11 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
         // points per round: as many as the job has, up to 64; halved while that lets one more CTA stay
         // on the SM (phases of different CTAs overlap) and each round still fills the MMA steps
         const int n_pts = d.Nchi * d.Neps;
-        auto layout = [&](int vs) {
+        auto layout = [&](int vs, int pad = 4, bool s_out = false) {
             ItemLayout y{};
             y.vs = vs;
-            y.ld = vs + 4;
+            y.ld = vs + pad;
+            y.s_out = s_out ? 2 * std::max(n_rows, 1) * NK : 0;
             y.parts = std::max(1, std::min(8, kItemThreads / (4 * vs)));
             size_t o = 0;
             y.y = o;
@@ -703,7 +710,7 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
             y.rv = o;
             o += (size_t)2 * NR * y.ld;
             y.s = o;
-            o += (size_t)2 * std::max(n_rows, 1) * NK;
+            o += s_out ? 0 : (size_t)2 * std::max(n_rows, 1) * NK;
             y.rl = o;
             o += (size_t)2 * NR;
             y.pts = o;
@@ -718,7 +725,11 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
         while (vs > 4 && layout(vs).total + 1024 > (size_t)max_smem) vs /= 2;
         while (vs > 16 && layout(vs).total > ((size_t)110 << 10)) vs /= 2;
         lay = layout(vs);
+        // operators whose tables do not fit so: columns without padding (bank conflicts), then S in device memory (any
+        // list of valid q, e.g. every q in every channel, or all harmonics at L = 23, K = 12)
+        for (int way = 1; way <= 2 && lay.total + 1024 > (size_t)max_smem; ++way) lay = layout(4, 0, way == 2);
         smem = lay.total;
+        if (lay.s_out) items = k_items<true>;
     }
     if (smem + 1024 > (size_t)max_smem) {
         cf_set_last_error("cf_rtensor_sumfac: N_Q too large for the shared-memory layout");
@@ -729,6 +740,7 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
     // within 48 MB, so they live in the 126 MB L2 between the two kernels instead of crossing HBM
     chunk = std::max<int64_t>(std::max<int64_t>(1, in->n_t2), ((int64_t)48 << 20) / ((int64_t)NL * 2 * NK * 8));
     chunk = std::min<int64_t>(chunk, n1 + j2 * std::max(in->n_t2, 0));
+    if (lay.s_out) chunk = std::min<int64_t>(chunk, ((int64_t)256 << 20) / ((int64_t)lay.s_out * 8));  // a CTA per item at most
     chunk = std::max<int64_t>(chunk, std::max<int64_t>(1, in->n_t2));
     n_split = std::max(1, std::min(64, (4 * n_sms + NL - 1) / NL));
     {
@@ -781,6 +793,7 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
         const size_t o_net = room((size_t)chunk * NL * 2 * NK), o_rad = room((size_t)chunk * 2 * NR);
         const size_t o_R = room(nR), o_part = room((size_t)n_split * nR);
         // the pair-major rows are read before the work buffers are written
+        const size_t o_s = room((size_t)chunk * lay.s_out);
         const size_t o_turn = pm ? room(std::max(ng1, ng2)) : 0;
         RT_CHECK(cudaMalloc((void**)&arena, total));
         for (auto& w : where) *w.first = arena + w.second;
@@ -792,6 +805,7 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
         radv = (double*)(arena + o_rad);
         dR = (double*)(arena + o_R);
         part = (double*)(arena + o_part);
+        s_scratch = (double*)(arena + o_s);
         turn = pm ? (double*)(arena + o_turn) : nullptr;
         RT_CHECK(cudaMemcpy(arena, small.data(), small.size(), cudaMemcpyHostToDevice));
         if (nl1) RT_CHECK(cudaMemcpy((double*)d.ploss1, in->p_loss_p1, nl1 * D, cudaMemcpyHostToDevice));
@@ -803,18 +817,13 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
             if (ns * ld == 0) continue;
             RT_CHECK(cudaMemcpy(pm ? turn : dgs[h], gs[h]->data, (size_t)ns * ld * D, cudaMemcpyHostToDevice));
             if (!pm) continue;
-            const int64_t gx = (ns + 31) / 32, gy = (ld + 31) / 32;
-            if (gy > 65535) {
-                cf_set_last_error("cf_rtensor_sumfac: too many (q, channel) pairs");
-                st = CF_ESHAPE;
-                goto done;
-            }
+            const int64_t gx = (ns + 31) / 32, gy = std::min<int64_t>(65535, (ld + 31) / 32);
             k_transpose<<<dim3((unsigned)gx, (unsigned)gy), 256>>>(turn, ld, ns, dgs[h]);
             RT_CHECK(cudaGetLastError());
         }
     }
     RT_CHECK(cudaMemset(part, 0, (size_t)n_split * nR * sizeof(double)));
-    RT_CHECK(cudaFuncSetAttribute(k_items, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RT_CHECK(cudaFuncSetAttribute(items, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     RT_CHECK(cudaEventCreate(&ev0));
     RT_CHECK(cudaEventCreate(&ev1));
     RT_CHECK(cudaEventRecord(ev0));
@@ -827,7 +836,7 @@ int sumfac_run(double* R_out, const cf_sumfac_inputs* in, const Channels& chn, c
         const int64_t here2 = ge - g0 - here1;
         const int64_t i0 = g0 < n1 ? g0 : n1 + (g0 - n1) * nt2, nc = here1 + here2 * nt2;
         const int64_t ctas = here1 + here2 * ((nt2 + kTBlock - 1) / kTBlock);
-        k_items<<<(unsigned)ctas, kItemThreads, smem>>>(d, lay, g0, ge - g0, i0, nc, net, radv);
+        items<<<(unsigned)ctas, kItemThreads, smem>>>(d, lay, g0, ge - g0, i0, nc, net, radv, s_scratch);
         RT_CHECK(cudaGetLastError());
         contract<<<dim3((unsigned)NL, (unsigned)n_split), kContractThreads>>>(d, net, radv, nc, part);
         RT_CHECK(cudaGetLastError());

@@ -414,13 +414,14 @@ __global__ void __launch_bounds__(1024) k_list(const int* __restrict__ active, i
     if (tid == 0) *count = done;
 }
 
-// Gather the listed cells of two tiled vectors into whole tiles (zeros past the last cell).
+// Gather the listed cells of two tiled vectors into whole tiles (zeros past the last cell); a block per tile in x, whose
+// number has no limit of 65535.
 __global__ void __launch_bounds__(256) k_gather(const double* __restrict__ a, const double* __restrict__ b,
                                                 double* __restrict__ ga, double* __restrict__ gb,
                                                 const int* __restrict__ list, int n, int M) {
-    const int lane = threadIdx.x & 31, tile = blockIdx.y, i = tile * kLanes + lane;
+    const int lane = threadIdx.x & 31, tile = blockIdx.x, i = tile * kLanes + lane;
     const size_t cell = i < n ? list[i] : 0, src = cell / kLanes * M * kLanes + cell % kLanes;
-    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < M; r += gridDim.x * 8) {
+    for (int r = blockIdx.y * 8 + (threadIdx.x >> 5); r < M; r += gridDim.y * 8) {
         const size_t dst = ((size_t)tile * M + r) * kLanes + lane;
         ga[dst] = i < n ? a[src + (size_t)r * kLanes] : 0.0;
         gb[dst] = i < n ? b[src + (size_t)r * kLanes] : 0.0;
@@ -563,7 +564,7 @@ extern "C" int cf_gmres_solve_tiled(cf_plan* plan, const double* f_t, double dt,
             if (few) {
                 double *fc = V + (size_t)(j + 2) * vec, *zc = fc + vec, *oc = zc + vec;
                 const int nt_c = (n_active + kLanes - 1) / kLanes;
-                k_gather<<<dim3((unsigned)std::min(64, (M + 7) / 8), (unsigned)nt_c), 256, 0, s>>>(f_t, z, fc, zc, list,
+                k_gather<<<dim3((unsigned)nt_c, (unsigned)std::min(64, (M + 7) / 8)), 256, 0, s>>>(f_t, z, fc, zc, list,
                                                                                                   n_active, M);
                 KLAUNCH();
                 rc = apply_J(oc, fc, zc, n_active);

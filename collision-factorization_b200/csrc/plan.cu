@@ -104,10 +104,10 @@ struct cf_plan {
     float* d_R32 = nullptr;  // FP32 copy of R for CF_FORM_AF_F32
     double* d_RT = nullptr;  // K = 8: R_t as [k1][8 k2 + k3] for the MMA kernel
     unsigned short* d_RTbf = nullptr;  // K = 8: the same split into BF16 hi and lo parts
-    int* d_x_q1 = nullptr;
-    int4* d_x_slice = nullptr;  // outer-product kernels' tables (build_outer)
+    double2* d_x_R = nullptr;  // outer-product kernels' tables (build_outer), one allocation
     unsigned char* d_x_chunk = nullptr;
-    double2* d_x_R = nullptr;
+    int4* d_x_slice = nullptr;
+    int* d_x_q1 = nullptr;
     int* d_item_q1 = nullptr;
     long long* d_item_cum = nullptr;
     int* d_bin_begin = nullptr;  // q1 bins of the tile kernel's work units (bin 0 = all, 1..4, 5..20)
@@ -285,11 +285,8 @@ void free_plan_memory(cf_plan* p) {
     cudaFree(p->d_R32);
     cudaFree(p->d_RT);
     cudaFree(p->d_RTbf);
-    cudaFree(p->d_x_q1);
-    cudaFree(p->d_item_cum);
-    cudaFree(p->d_x_slice);
-    cudaFree(p->d_x_chunk);
     cudaFree(p->d_x_R);
+    cudaFree(p->d_item_cum);
     cudaFree(p->d_item_q1);
     cudaFree(p->d_bin_begin);
     cudaFree(p->d_bin_q1);
@@ -314,121 +311,58 @@ void free_plan_memory(cf_plan* p) {
         if (hs) cudaStreamDestroy(hs);
 }
 
-// Tables of the outer-product kernels (outer_kernels.cuh): every slice's entries as runs of equal q2 of one
-// or two entries, four runs to a chunk, the runs of two first.  Runs of a chunk are picked so that
-// their q2, and their q3 of either column, are distinct modulo 4 as far as a few candidates allow (the
-// operands of eight lanes then lie in distinct banks: 20 % above the conflict-free count at L = 10, 39 %
-// in the list's own order).
+// Tables of the outer-product kernels (outer_kernels.cuh).  The host counts every slice's runs (equal q2, one or two
+// entries) and places its chunks of four; the chunks themselves are packed on the device (pack_chunks_kernel), as
+// every plan has them made, also one whose fast forms are never called: a plan's making takes 4.2 ms at L = 10, K = 8 and
+// 8.8 at L = 13 (packed on the host 5.3 and 14.4; without these tables, and all copies of R made on the host, 4.2 and 10.0).
 int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<int>& slice_t,
-                const std::vector<int>& slice_e, const std::vector<uint32_t>& e_q23, const std::vector<double>& e_g,
-                int64_t& bytes) {
-    constexpr size_t kLook = 6;  // candidates per place
-    struct Run {
-        unsigned short q2, qa, qb, two;
-        double ga, gb;
-    };
-    struct Chunk {
-        ushort4 q[4];
-        double2 g[4];
-    };
-    static_assert(sizeof(Chunk) == 96, "the kernels copy chunks of 96 bytes");
+                const std::vector<int>& slice_e, const std::vector<uint32_t>& e_q23, int64_t& bytes) {
     const size_t S = slice_t.size();
-    std::vector<int4> xs;
-    std::vector<int> xbegin(S + 1, 0), xq1(q1_begin.size());
-    std::vector<unsigned char> xb;
+    std::vector<int4> xs, place(S);  // place: first chunk, runs of two, runs
+    std::vector<int> xbegin(S + 1, 0), xq1(q1_begin.size()), count(p->n_q, 0);
     xs.reserve(S + S / 8);
-    xb.reserve((e_q23.size() / 3 + S) * sizeof(Chunk));
-    const int n_zero = cf::outer_zeros(p->n_q, cf::outer_nqp(cf::outer_fit(p->n_q, p->k, false, p->max_smem).width));
-    std::vector<uint64_t> ent;  // q2 << 32 | entry
-    std::vector<Run> all, one;
-    size_t n_chunks = 0;
+    int n_chunks = 0;
     for (size_t s = 0; s < S; ++s) {
-        ent.clear();
-        bool sorted = true;
+        for (int e = slice_e[s]; e < slice_e[s + 1]; ++e) ++count[e_q23[e] & 0xffffu];
+        int n_two = 0, n_all = 0;
         for (int e = slice_e[s]; e < slice_e[s + 1]; ++e) {
-            const uint64_t x = (uint64_t)(e_q23[e] & 0xffffu) << 32 | (uint64_t)e;
-            sorted = sorted && (ent.empty() || ent.back() < x);
-            ent.push_back(x);
+            int& c = count[e_q23[e] & 0xffffu];
+            n_two += c / 2;
+            n_all += (c + 1) / 2;
+            c = 0;
         }
-        if (!sorted) std::sort(ent.begin(), ent.end());
-        all.clear();
-        one.clear();
-        for (size_t i = 0; i < ent.size();) {
-            const bool two = i + 1 < ent.size() && ent[i + 1] >> 32 == ent[i] >> 32;
-            const uint32_t ea = (uint32_t)ent[i], eb = two ? (uint32_t)ent[i + 1] : ea;
-            (two ? all : one).push_back({(unsigned short)(ent[i] >> 32), (unsigned short)(e_q23[ea] >> 16),
-                                         (unsigned short)(e_q23[eb] >> 16), two, e_g[ea], two ? e_g[eb] : 0.0});
-            i += two ? 2 : 1;
-        }
-        const size_t n_two = all.size();
-        all.insert(all.end(), one.begin(), one.end());
-        const int begin = (int)n_chunks;
-        for (size_t i0 = 0; i0 < all.size(); i0 += 4) {
-            int used[3][4] = {};  // residues taken in this chunk: q2, q3a, q3b
-            const bool two = i0 < n_two;  // the kernel reads q3b too
-            for (size_t i = i0; i < std::min(i0 + 4, all.size()); ++i) {
-                const size_t hi = std::min(i + kLook, i < n_two ? n_two : all.size());  // runs of two stay in front
-                size_t best = i;
-                bool flip = false;
-                int c_best = 1 << 20;
-                for (size_t c = i; c < hi && c_best > 0; ++c) {
-                    const Run& r = all[c];
-                    const int c2 = used[0][r.q2 & 3], a0 = used[1][r.qa & 3] + used[2][r.qb & 3],
-                              a1 = used[1][r.qb & 3] + used[2][r.qa & 3];
-                    if (c2 + std::min(a0, a1) < c_best) {
-                        c_best = c2 + std::min(a0, a1);
-                        best = c;
-                        flip = r.two && a1 < a0;
-                    }
-                }
-                if (best != i) std::swap(all[i], all[best]);
-                Run& r = all[i];
-                if (flip) {
-                    std::swap(r.qa, r.qb);
-                    std::swap(r.ga, r.gb);
-                }
-                ++used[0][r.q2 & 3];
-                ++used[1][r.qa & 3];
-                ++used[2][r.qb & 3];
-            }
-            // the row of zeros in the residue that the fewest others of its kind have
-            auto zero_row = [&](int kind) {
-                int best = 0;
-                for (int z = 1; z < n_zero; ++z)
-                    if (used[kind][(p->n_q + z) & 3] < used[kind][(p->n_q + best) & 3]) best = z;
-                ++used[kind][(p->n_q + best) & 3];
-                return (unsigned short)(16 * (p->n_q + best));
-            };
-            Chunk c;
-            for (size_t i = 0; i < 4; ++i) {
-                // as byte offsets in a row of cell pairs (N_Q < 268 where the kernels run)
-                if (i0 + i < all.size()) {
-                    const Run& r = all[i0 + i];
-                    c.q[i] = make_ushort4((unsigned short)(16 * r.q2), (unsigned short)(16 * r.qa),
-                                          r.two || !two ? (unsigned short)(16 * r.qb) : zero_row(2), 0);
-                    c.g[i] = make_double2(r.ga, r.gb);
-                } else {
-                    c.q[i] = make_ushort4(zero_row(0), zero_row(1), zero_row(2), 0);
-                    c.g[i] = make_double2(0.0, 0.0);
-                }
-            }
-            xb.insert(xb.end(), (const unsigned char*)&c, (const unsigned char*)(&c + 1));
-            ++n_chunks;
-        }
+        place[s] = make_int4(n_chunks, n_two, n_all, 0);
         // a ring stage holds kOuterChunks chunks; the K^3 step is linear, so a longer slice is several
-        const int n = (int)((all.size() + 3) / 4), n2 = (int)((n_two + 3) / 4);
+        const int n = (n_all + 3) / 4, n2 = (n_two + 3) / 4;
         for (int c = 0; c < n; c += cf::kOuterChunks)
-            xs.push_back(make_int4(slice_t[s], begin + c, std::max(0, std::min(cf::kOuterChunks, n2 - c)),
+            xs.push_back(make_int4(slice_t[s], n_chunks + c, std::max(0, std::min(cf::kOuterChunks, n2 - c)),
                                    std::min(cf::kOuterChunks, n - c)));
+        n_chunks += n;
         xbegin[s + 1] = (int)xs.size();
     }
     for (size_t q = 0; q < q1_begin.size(); ++q) xq1[q] = xbegin[q1_begin[q]];
-    CF_TRY(upload(&p->d_x_q1, xq1, bytes));
-    CF_TRY(upload(&p->d_x_slice, xs, bytes));
-    CF_TRY(upload(&p->d_x_chunk, xb, bytes));
-    const size_t nR = (size_t)p->n_l * p->k * 32;
-    CF_CUDA(cudaMalloc((void**)&p->d_x_R, std::max<size_t>(nR, 1) * sizeof(double2)));
-    bytes += (int64_t)(nR * sizeof(double2));
+    // one allocation: R_t in lane order, the chunks, then what the host made
+    const size_t nR = (size_t)p->n_l * p->k * 32, b_R = nR * sizeof(double2), b_ch = (size_t)n_chunks * cf::kOuterChunkWords * 8;
+    const size_t b_xs = xs.size() * sizeof(int4), b_pl = S * sizeof(int4), b_q1 = xq1.size() * sizeof(int);
+    std::vector<unsigned char> host(b_xs + b_pl + b_q1);
+    if (b_xs) std::memcpy(host.data(), xs.data(), b_xs);
+    if (b_pl) std::memcpy(host.data() + b_xs, place.data(), b_pl);
+    std::memcpy(host.data() + b_xs + b_pl, xq1.data(), b_q1);
+    unsigned char* d = nullptr;
+    CF_CUDA(cudaMalloc((void**)&d, b_R + b_ch + host.size()));
+    p->d_x_R = (double2*)d;
+    p->d_x_chunk = d + b_R;
+    p->d_x_slice = (int4*)(d + b_R + b_ch);
+    const int4* d_place = p->d_x_slice + xs.size();
+    p->d_x_q1 = (int*)(d_place + S);
+    bytes += (int64_t)(b_R + b_ch + host.size());
+    CF_CUDA(cudaMemcpy(d + b_R + b_ch, host.data(), host.size(), cudaMemcpyHostToDevice));
+    const int n_zero = cf::outer_zeros(p->n_q, cf::outer_nqp(cf::outer_fit(p->n_q, p->k, false, p->max_smem).width));
+    if (S > 0) {
+        cf::pack_chunks_kernel<<<(unsigned)((S + 63) / 64), 64>>>(p->d_slice_e, p->d_e_q23, p->d_e_g, d_place, (int)S, p->n_q,
+                                                                 n_zero, (unsigned long long*)p->d_x_chunk);
+        CF_CUDA(cudaGetLastError());
+    }
     if (nR > 0) {
         cf::lane_order_kernel<<<(unsigned)((nR + 255) / 256), 256>>>(p->d_R, p->d_x_R, nR, p->k);
         CF_CUDA(cudaGetLastError());
@@ -604,7 +538,7 @@ int build_plan(cf_plan* p, const double* labels, const double* vals, const doubl
     CF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     p->max_smem = (size_t)optin;
     if (cf::outer_for(K) && cf::outer_fit(NQ, K, false, p->max_smem).nc > 0)
-        CF_TRY(build_outer(p, q1_begin, slice_t, slice_e, e_q23, e_g, bytes));
+        CF_TRY(build_outer(p, q1_begin, slice_t, slice_e, e_q23, bytes));
     CF_CUDA(cudaStreamSynchronize(nullptr));  // a launch on another stream may read what the kernels here wrote
     p->dev_bytes = bytes;
     return CF_OK;

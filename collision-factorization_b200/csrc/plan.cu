@@ -313,8 +313,8 @@ void free_plan_memory(cf_plan* p) {
 
 // Tables of the outer-product kernels (outer_kernels.cuh).  The host counts every slice's runs (equal q2, one or two
 // entries) and places its chunks of four; the chunks themselves are packed on the device (pack_chunks_kernel), as
-// every plan has them made, also one whose fast forms are never called: a plan's making takes 4.2 ms at L = 10, K = 8 and
-// 8.8 at L = 13 (packed on the host 5.3 and 14.4; without these tables, and all copies of R made on the host, 4.2 and 10.0).
+// every plan has them made, also one whose fast forms are never called: a plan's making takes 3.5 ms at L = 10, K = 8
+// (packed on one host thread 5.0; without these tables, and all copies of R made on the host, 3.8).
 int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<int>& slice_t,
                 const std::vector<int>& slice_e, const std::vector<uint32_t>& e_q23, int64_t& bytes) {
     const size_t S = slice_t.size();

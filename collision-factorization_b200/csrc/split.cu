@@ -1006,6 +1006,29 @@ __device__ __forceinline__ void lb_dmma(double& d0, double& d1, double a, double
                  : "d"(a), "d"(b));
 }
 
+// The run records of an item, a thread each; src: its entries (begin, end) and the q of the stage's first row as band l2
+// and as band l3 see it.
+__global__ void __launch_bounds__(64) lb_records_kernel(const int4* __restrict__ items, const int4* __restrict__ src, int n_items,
+                                                        const uint32_t* __restrict__ e_q23, const double* __restrict__ e_g,
+                                                        int row_bytes, uint4* __restrict__ recs, uint4* __restrict__ recs32) {
+    const int i = blockIdx.x * 64 + threadIdx.x;
+    if (i >= n_items) return;
+    const int4 s = src[i];
+    int run = items[i].z;
+    for (int z = s.x; z < s.y; ++run) {
+        const uint32_t a = e_q23[z];
+        const bool two = z + 1 < s.y && ((a ^ e_q23[z + 1]) & 0xffffu) == 0;
+        const uint32_t b = two ? e_q23[z + 1] : a;
+        const double ga = two ? e_g[z] : 0.5 * e_g[z], gb = two ? e_g[z + 1] : ga;
+        const uint32_t o2 = ((int)(a & 0xffffu) - s.z) * row_bytes, oa = ((int)(a >> 16) - s.w) * row_bytes,
+                       ob = ((int)(b >> 16) - s.w) * row_bytes;
+        recs[2 * (size_t)run] = make_uint4(__double2loint(ga), __double2hiint(ga), __double2loint(gb), __double2hiint(gb));
+        recs[2 * (size_t)run + 1] = make_uint4(o2, oa, ob, 0u);
+        recs32[run] = make_uint4(__float_as_uint((float)ga), __float_as_uint((float)gb), o2, oa / 16 | ob / 16 << 16);
+        z += two ? 2 : 1;
+    }
+}
+
 enum { LBI_TR = 0, LBI_ORD, LBI_BEGIN, LBI_END };  // item: t | row << 16, ord, its run records
 enum { LBU_L1 = 0, LBU_BROWS, LBU_TLOFF, LBU_NT, LBU_ITOFF, LBU_NIT, LBU_INTS = 8 };
 
@@ -1706,6 +1729,29 @@ void split_r_bf16(const std::vector<double>& R, int n_l, std::vector<uint8_t>& p
     }
 }
 
+// The run records, made on the device from the operator's entries.  First call at L = 16, K = 12, which makes the tables:
+// plain 97 ms, folded with the folding 137 (with the records made on the host 123 and 145).
+cudaError_t make_records(SplitPlan* sp, const DevOp& op, const std::vector<int4>& src, int n_recs, int k, int64_t& bytes) {
+    int4* d_src = nullptr;
+    int64_t scratch = 0;
+    cudaError_t e = upload_vec(&d_src, src, scratch);
+    const size_t n = std::max(n_recs, 1);
+    if (e == cudaSuccess) e = cudaMalloc(&sp->d_lb_recs, n * 32);
+    if (e == cudaSuccess) e = cudaMalloc(&sp->d_lb_recs32, n * 16);
+    if (e == cudaSuccess && !src.empty()) {
+        lb_records_kernel<<<(unsigned)((src.size() + 63) / 64), 64>>>(sp->d_lb_items, d_src, (int)src.size(), op.e_q23, op.e_g,
+                                                                     k * kLbCells * (int)sizeof(double), sp->d_lb_recs,
+                                                                     sp->d_lb_recs32);
+        e = cudaGetLastError();
+        // launches on other streams read the records
+        const cudaError_t e2 = cudaStreamSynchronize(nullptr);
+        if (e == cudaSuccess) e = e2;
+    }
+    cudaFree(d_src);
+    bytes += (int64_t)n * 48;
+    return e;
+}
+
 template <int K, int C>
 int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
     using S = Shape<K, C>;
@@ -1859,20 +1905,9 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
     // its row's slices (the row's ticket) and the (l2, l3) of its t
     std::vector<int> units_lb, order_lb, titems_lb(band_tl.size(), 0);
     std::vector<int4> items_lb;
-    std::vector<uint4> recs64, recs32;  // run records (LbRun), two words of 16 bytes per run in FP64
+    std::vector<int4> rec_src;  // per item: its entries (begin, end), first q of its stage's rows (lb_records_kernel)
+    int n_recs = 0;
     std::vector<double> work_lb;
-    constexpr uint32_t kRowB = K * kLbCells * sizeof(double);  // = K 16 sizeof(float)
-    auto add_run = [&](double ga, double gb, uint32_t r2, uint32_t r3a, uint32_t r3b) {
-        uint32_t g[4];
-        std::memcpy(g, &ga, 8);
-        std::memcpy(g + 2, &gb, 8);
-        recs64.push_back(make_uint4(g[0], g[1], g[2], g[3]));
-        recs64.push_back(make_uint4(r2 * kRowB, r3a * kRowB, r3b * kRowB, 0u));
-        const float fa = (float)ga, fb = (float)gb;
-        std::memcpy(g, &fa, 4);
-        std::memcpy(g + 1, &fb, 4);
-        recs32.push_back(make_uint4(g[0], g[1], r2 * kRowB, (r3a * kRowB / 16) | (r3b * kRowB / 16) << 16));
-    };
     int lb_rows = 0, lb_t = 0;
     bool lb_ok = L < 128;
     for (const BandInfo& bd : bands) {
@@ -1882,21 +1917,15 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
             const int t = band_tl[bd.tl_off + ti];
             const int l2 = t_l23[t] & 0xff, l3 = t_l23[t] >> 8;
             // first q of the stage's rows: band l2, then (unless it is the same) band l3
-            const uint32_t b2 = l2 * l2, b3 = l3 * l3 - (l3 != l2 ? 2 * l2 + 1 : 0);
+            const int b2 = l2 * l2, b3 = l3 * l3 - (l3 != l2 ? 2 * l2 + 1 : 0);
             for (int r = 0; r < bd.brows; ++r) {
                 const int sl = band_slice[bd.tab_off + (size_t)ti * bd.brows + r];
                 if (sl < 0) continue;
-                const int run0 = (int)(recs32.size());
-                if (lblock_supported_k(K))
-                    for (int z = slice_e[sl]; z < slice_e[sl + 1];) {
-                        const uint32_t q2 = e_q23[z] & 0xffffu, q3 = e_q23[z] >> 16;
-                        const bool two = z + 1 < slice_e[sl + 1] && (e_q23[z + 1] & 0xffffu) == q2;
-                        const double g = two ? e_g[z] : 0.5 * e_g[z];
-                        add_run(g, two ? e_g[z + 1] : g, q2 - b2, q3 - b3,
-                                (two ? e_q23[z + 1] >> 16 : q3) - b3);
-                        z += two ? 2 : 1;
-                    }
-                items_lb.push_back(make_int4(ti | (r << 16), ord[r]++, run0, (int)recs32.size()));
+                const int run0 = n_recs, z1 = slice_e[sl + 1];
+                for (int z = slice_e[sl]; lblock_supported_k(K) && z < z1; ++n_recs)
+                    z += z + 1 < z1 && ((e_q23[z] ^ e_q23[z + 1]) & 0xffffu) == 0 ? 2 : 1;
+                rec_src.push_back(make_int4(slice_e[sl], z1, b2, b3));
+                items_lb.push_back(make_int4(ti | (r << 16), ord[r]++, run0, n_recs));
                 ++titems_lb[bd.tl_off + ti];
             }
         }
@@ -1995,9 +2024,8 @@ int build_impl(SplitPlan* sp, const DevOp& op, int64_t n_g, int64_t n_slices) {
         (ce = upload_vec(&sp->d_lb_order, order_lb, bytes)) != cudaSuccess ||
         (ce = upload_vec(&sp->d_lb_items, items_lb, bytes)) != cudaSuccess ||
         (ce = upload_vec(&sp->d_lb_titems, titems_lb, bytes)) != cudaSuccess ||
-        (ce = upload_vec(&sp->d_lb_recs, recs64, bytes)) != cudaSuccess ||
-        (ce = upload_vec(&sp->d_lb_recs32, recs32, bytes)) != cudaSuccess ||
-        (ce = upload_vec(&sp->d_t_l23, t_l23, bytes)) != cudaSuccess)
+        (ce = upload_vec(&sp->d_t_l23, t_l23, bytes)) != cudaSuccess ||
+        (lblock_supported_k(K) && (ce = make_records(sp, op, rec_src, n_recs, K, bytes)) != cudaSuccess))
         return fail_split(ce == cudaErrorMemoryAllocation ? CF_ENOMEM : CF_ECUDA,
                           std::string("split form: upload: ") + cudaGetErrorString(ce));
     sp->bytes = bytes;

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import argparse
 import concurrent.futures as cf
+import hashlib
 import os
 import shutil
 import subprocess
@@ -38,6 +39,14 @@ def _deps() -> list[Path]:
     return sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh")) + [INCLUDE / "cf_b200.h"]
 
 
+def source_id() -> str:
+    """Digest of the library's sources; cf_version() carries it."""
+    h = hashlib.sha256()
+    for p in _deps():
+        h.update(p.name.encode() + b"\0" + p.read_bytes())
+    return h.hexdigest()[:12]
+
+
 def _stale(obj: Path) -> bool:
     if not obj.exists():
         return True
@@ -57,7 +66,7 @@ def _compile(src: Path, obj: Path, defines: list[str]) -> tuple[Path, str]:
 
 def build(force: bool = False, jobs: int | None = None, verbose: bool = True) -> Path:
     BUILD.mkdir(exist_ok=True)
-    units = [(CSRC / "plan.cu", BUILD / "plan.o", []), (CSRC / "noalloc.cu", BUILD / "noalloc.o", []),
+    units = [(CSRC / "plan.cu", BUILD / "plan.o", [f'-DCF_SOURCE_ID="{source_id()}"']), (CSRC / "noalloc.cu", BUILD / "noalloc.o", []),
              (CSRC / "krylov.cu", BUILD / "krylov.o", []), (CSRC / "mlp.cu", BUILD / "mlp.o", []),
              (CSRC / "ragged.cu", BUILD / "ragged.o", []), (CSRC / "stepping.cu", BUILD / "stepping.o", []),
              (CSRC / "rtensor.cu", BUILD / "rtensor.o", []), (CSRC / "split.cu", BUILD / "split.o", []),

@@ -2251,6 +2251,10 @@ const char* cf_status_string(int status) {
 const char* cf_last_error(void) { return g_last_error.c_str(); }
 int64_t cf_launch_count(void) { return g_launches.load(); }
 int cf_few_route_last(void) { return g_few_route; }
-const char* cf_version(void) { return "cf_b200 0.1 (sm_100a)"; }
+// The sources' digest (set by build.py) is part of it: the autotuners' caches hold a choice for one set of kernels.
+#ifndef CF_SOURCE_ID
+#define CF_SOURCE_ID "unknown"
+#endif
+const char* cf_version(void) { return "cf_b200 0.2 (sm_100a, kernels " CF_SOURCE_ID ")"; }
 
 }  // extern "C"

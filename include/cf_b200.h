@@ -405,7 +405,8 @@ int64_t cf_launch_count(void);
  * few-cell kernel, 1 f and Q_in in the launch's parameter block (Q_out written to mapped pinned
  * memory), 2 copies through pinned staging and a device buffer. */
 int cf_few_route_last(void);
-/* Library version string. */
+/* Library version string, with a digest of the kernels' sources: what was measured with one version (the
+ * autotuners' caches) is not taken over by another. */
 const char* cf_version(void);
 
 #ifdef __cplusplus

@@ -447,12 +447,12 @@ def run_ours(args):
     err_sym = form_err()
     sym_ms = timed(lambda: step("af_sym"), args.steps)
     sym_kern_ms = timed(lambda: kernel_only("af_sym"), max(2, args.steps // 2))
-    # the folded form's device step is one launch of the tile kernel on the cell-major arrays (no
-    # layout passes) when it runs on the tile kernel: then that launch is the roofline kernel
+    # the folded form's device step is one launch on the cell-major arrays (no layout passes) when it runs on the
+    # tile or the outer-product kernel: then that launch is the roofline kernel
     n0 = _lib.launch_count()
     op.q(f, out=Q, form="af_sym", workspace=ws)
     torch.cuda.synchronize(dev)
-    sym_single = _lib.launch_count() - n0 == 1 and _lib.PATH_NAMES[op.info()["last_path"]] == "tile"
+    sym_single = _lib.launch_count() - n0 == 1 and op.last_kernel() in ("tile", "outer", "outer_8")
     if sym_single:
         sym_kern_ms = timed(lambda: op.q(f, out=Q, form="af_sym", workspace=ws), max(2, args.steps // 2))
     path_ms, sym_path_ms = {}, {}
@@ -527,7 +527,7 @@ def run_ours(args):
     n0 = _lib.launch_count()
     step(chosen)
     torch.cuda.synchronize(dev)
-    step_path = _lib.PATH_NAMES[op.info()["last_path"]]
+    step_path = op.last_kernel()
     step_launches = _lib.launch_count() - n0
     if ((step_path in ("split_i8", "band") and step_launches == 1) or step_path == "rf_dense"
             or (step_path == "lblock" and step_launches == 2)):
@@ -537,11 +537,9 @@ def run_ours(args):
         kern_list = sym_kern_ms if chosen == "af_sym" else kern_ms
         kernel_only(chosen)
         torch.cuda.synchronize(dev)
-        last_path = _lib.PATH_NAMES[op.info()["last_path"]]
-        if chosen == "af_sym" and sym_single:
+        last_path = op.last_kernel()
+        if chosen == "af_sym" and sym_single and last_path == "tile":
             last_path = "tile_cell_major"
-        if K in (7, 8) and last_path in ("tile", "tile_cell_major") and args.path in (None, "auto"):
-            last_path = "outer"
     traffic = NCU_TRAFFIC.get((args.workload, last_path, chosen))
     kern_name = {"pair": "af_pair_kernel (persistent, tile-resident, mirrored row pairs)",
                  "pair_split": "af_pair_kernel, split variant (both mirrored rows per lane, k3 halves)",
@@ -549,6 +547,7 @@ def run_ours(args):
                  "tile_cell_major": "af_tile_kernel on the cell-major arrays (no layout passes; the whole device step)",
                  "outer": "af_outer_kernel (Phi on the FP64 tensor cores, four runs of equal q2 per mma.sync m8n8k4; on the "
                           "cell-major arrays; the whole device step)",
+                 "outer_8": "af_outer_kernel on units of 8 cells",
                  "gather": "af_kernel (gathers through L1/L2)",
                  "tile_mma": "af_mma_kernel (tile-resident, K^3 step on the FP64 MMA)",
                  "split_i8": "af_split_kernel (Phi in FP64 on the folded operator, K^3 step on the int8 tensor cores "
@@ -1362,7 +1361,7 @@ def run_single(args):
         torch.cuda.synchronize(dev)
         per_form[form] = {"device_us": median_us(dev_s), "device_us_mean": 1e6 * sum(dev_s) / len(dev_s),
                           "round_trip_us": median_us(round_trip(lambda: call(form), steps)),
-                          "launches_per_call": launches, "path": _lib.PATH_NAMES.get(op.info()["last_path"], "?")}
+                          "launches_per_call": launches, "path": op.last_kernel()}
     # floors: one empty launch (a 1-element fill) and the copies of one f
     one = torch.zeros(1, dtype=torch.float64, device=dev)
     floor_launch = median_us(round_trip(lambda: one.fill_(1.0), steps))

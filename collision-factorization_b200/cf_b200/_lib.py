@@ -31,7 +31,7 @@ FORMS = {"af": FORM_AF, "rf": FORM_RF, "af_exact": FORM_AF_EXACT, "rf_exact": FO
 # Every symbol the header declares; the tests check that the library exports all of them.
 EXPORTS = [
     "cf_angular_first", "cf_radial_first", "cf_contract_host", "cf_time_contract_host", "cf_jacobian_apply_host",
-    "cf_plan_create", "cf_plan_destroy", "cf_plan_get_info", "cf_plan_workspace_size",
+    "cf_plan_create", "cf_plan_destroy", "cf_plan_get_info", "cf_plan_last_kernel", "cf_plan_workspace_size",
     "cf_q_device", "cf_q_device_ws", "cf_jv_device", "cf_q_device_noalloc", "cf_plan_stream_selftest",
     "cf_plan_lblock_selftest",
     "cf_ragged_create", "cf_ragged_destroy", "cf_ragged_q", "cf_ragged_graph_launch", "cf_ragged_q_resident",
@@ -148,6 +148,8 @@ def load(path: str | Path | None = None) -> C.CDLL:
     lib.cf_launch_count.restype = C.c_int64
     lib.cf_few_route_last.restype = C.c_int
     lib.cf_version.restype = C.c_char_p
+    lib.cf_plan_last_kernel.restype = C.c_char_p
+    lib.cf_plan_last_kernel.argtypes = [C.c_void_p]
     if path is None:
         _lib = lib
     return lib

@@ -123,6 +123,11 @@ class CollisionOperator:
         _lib.check(_lib.load().cf_plan_get_info(self._h, C.byref(inf)))
         return {f: getattr(inf, f) for f, _ in inf._fields_}
 
+    def last_kernel(self) -> str:
+        """The kernel of the last angular-first or J.v launch by name ('outer' and 'outer_8' for the
+        outer-product kernel, which info()['last_path'] reports as the tile kernels' codes)."""
+        return _lib.load().cf_plan_last_kernel(self._h).decode()
+
     def content_digest(self) -> str:
         """SHA-256 (hex, 16 chars) of the operator's arrays: names the operator in caches."""
         if not hasattr(self, "_digest"):

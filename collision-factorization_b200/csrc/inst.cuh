@@ -194,7 +194,7 @@ static inline UnitPlan plan_units(int64_t n_cells, int64_t ctas) {
 template <int K, bool JV>
 static LaunchResult launch_outer(const LaunchArgs& a) {
     const OuterFit fit = outer_fit(a.op.n_q, K, JV, a.max_smem);
-    const int path = fit.nc == 16 ? PATH_TILE : PATH_TILE4;
+    const int path = fit.nc == 16 ? PATH_OUTER : PATH_OUTER8;
     const bool stream = a.ss && a.ss->ready;
     if (a.op.x_slice == nullptr || a.op.n_items == 0 || a.counter == nullptr || fit.nc == 0 || (stream && fit.nc != 16))
         return {-1, 0, cudaSuccess, path};

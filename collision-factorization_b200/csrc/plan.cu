@@ -1971,9 +1971,19 @@ int cf_plan_get_info(const cf_plan* plan, cf_plan_info* info) {
     info->flops_q = plan->flops_q;
     info->flops_jv = plan->flops_jv;
     info->device_bytes = plan->dev_bytes + (int64_t)plan->ws_bytes + (int64_t)plan->io_bytes;
-    info->last_path = plan->last_path;
+    info->last_path = plan->last_path == cf::PATH_OUTER    ? (int)cf::PATH_TILE
+                      : plan->last_path == cf::PATH_OUTER8 ? (int)cf::PATH_TILE4
+                                                           : plan->last_path;
     info->reserved = 0;
     return CF_OK;
+}
+
+const char* cf_plan_last_kernel(const cf_plan* plan) {
+    static const char* const names[] = {"none", "gather", "tile", "pair", "pair_l1", "pair_split", "tile_mma", "bf16_mma",
+                                        "tile_quarter", "few", "split_i8", "band", "band_bf16", "rf_dense", "lblock",
+                                        "outer", "outer_8"};
+    static_assert(sizeof(names) / sizeof(names[0]) == cf::PATH_OUTER8 + 1, "a name per path");
+    return plan ? names[plan->last_path] : "none";
 }
 
 int cf_plan_workspace_size(const cf_plan* plan, int64_t b, int32_t jacobian, size_t* bytes) {

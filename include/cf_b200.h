@@ -159,6 +159,9 @@ int cf_plan_create(cf_plan** plan, const double* labels, const double* vals, con
                    int32_t device);
 int cf_plan_destroy(cf_plan* plan);
 int cf_plan_get_info(const cf_plan* plan, cf_plan_info* info);
+/* The kernel of the plan's last angular-first or J.v launch by name: "none", "gather", "tile", "pair", ... as in last_path,
+ * and "outer" or "outer_8" (units of 16 or 8 cells) for the outer-product kernel, which last_path reports as 2 or 8. */
+const char* cf_plan_last_kernel(const cf_plan* plan);
 
 /* Bytes of device scratch the batched calls need for B cells (the tiled copies of the inputs
  * and of the output).  Passing a workspace of at least this size to the *_ws calls makes

@@ -19,7 +19,9 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <thread>
 #include <vector>
 
@@ -174,8 +176,8 @@ struct RaggedSync {
 // Resident (rs.ready null; the device steps): the same routine on the callers' cell-major arrays in
 // `ptrs`, no waits and no chunk words -- the whole step in one launch, without layout passes.  Its table
 // (`groups`) gives the warps several half-tiles at a time where one has few rows, heaviest rows first
-// (a half-tile at L = 4 has 25 rows for 16 warps), and cuts those that would outlast a CTA's share of the work: a whole
-// one at L = 10, K = 8 takes 0.95 ms.  B200, L, K = 4, 4; 6, 6; 8, 6; 10, 8 at 40, 30, 20, 10 % of the cells, against whole
+// (a half-tile at L = 4 has 25 rows for 16 warps), and cuts those that would outlast a CTA's share of the work (a whole
+// one at L = 10, K = 8 takes 0.95 ms) or, where that is the shorter by estimate, the last ones.  B200, L, K = 4, 4; 6, 6; 8, 6; 10, 8 at 40, 30, 20, 10 % of the cells, against whole
 // half-tiles and quarters of as many as there are CTAs at the end: 600 cells 284 -> 135 us, 2500: 978 -> 278, 6000: 986 ->
 // 523, 10000: 982 -> 814, 16384: 1298 -> 1293.
 __global__ void __launch_bounds__(kTW * 32, 1)
@@ -831,11 +833,32 @@ int cf_ragged_create(cf_ragged** out, cf_plan* const* plans, const int64_t* cell
         r->cell_major = cm;
         std::vector<Unit> groups;
         if (cm) {
-            // A CTA's share of the work decides: a half-tile of more than 0.8 of it is taken in tail_split parts, or
-            // where a quarter is still more than two shares in 16 (some 8 rows for 16 warps, but a heavy row alone is half a
-            // quarter's time), and light ones together, as many as give 6 rows a
-            // warp, fit where the largest bucket's one fits and are at most 0.03 of a share.
             auto cost = [&](int b) { return r->cost[b] * (1.0 + 25.0 / (r->K[b] * r->K[b])); };  // FLOPs, and more per FLOP at small K
+            // A table's time, its units taken in order by the CTAs as they come free.  A unit: its rows in rounds of 16 (a
+            // lone row takes 0.7 of a round's time), a third of a round lost at its end, and 8 us (2.8e6 of cost) of
+            // staging.  Within 10 % of what was measured for nine in ten of 38 mixes and sizes (sixteenths at K = 4 take less).
+            auto time_of = [&](const std::vector<Unit>& table) {
+                std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+                double last = 0.0;
+                for (const Unit& u : table) {
+                    const double rows = std::max(1, hb[u.bucket].op.n_items), parts = u.bin == 0 ? 1 : u.bin <= 4 ? 4 : 16;
+                    double t = cost(u.bucket) / rows * kTW * (std::max(rows * u.chunk / parts / kTW, 0.35) + 0.35) + 2.8e6;
+                    if ((int)free_at.size() == r->ctas) {
+                        t += free_at.top();
+                        free_at.pop();
+                    }
+                    free_at.push(t);
+                    last = std::max(last, t);
+                }
+                return last;
+            };
+            // Either a CTA's share of the work decides: a half-tile of more than 0.8 of it is taken in tail_split parts, or
+            // where a quarter is still more than two shares in 16 (some 8 rows for 16 warps, but a heavy row alone is half a
+            // quarter's time), and light ones together, as many as give 6 rows a warp, fit where the largest bucket's
+            // one fits and are at most 0.03 of a share.  Or the last half-tiles of the work table are cut, as many as there
+            // are CTAs: better where a few rounds of whole ones would end in a nearly empty one (B200, us, by share / last
+            // cut): L = 8, K = 8, 3000 cells 791 / 621, 8000 cells 1565 / 1454; L, K = 4, 4; 6, 6; 8, 6; 10, 8 at a quarter each, 8000
+            // cells, tail_split 16 1683 / 1255; 4, 4 and 10, 8 at 95 and 5 %, 8000 cells 268 / 963.
             double share = 0.0;
             for (const auto& h : hts) share += cost(h.first) / r->ctas;
             for (size_t i = 0; i < n_ht;) {
@@ -852,6 +875,9 @@ int cf_ragged_create(cf_ragged** out, cf_plan* const* plans, const int64_t* cell
                 }
                 i += n;
             }
+            std::vector<Unit> last_cut = units;
+            for (Unit& u : last_cut) u.chunk = 1;
+            if (time_of(last_cut) < 0.985 * time_of(groups)) groups = last_cut;
             r->n_groups = (int)groups.size();
         }
         e = cudaMalloc(&r->d_tiles, std::max<size_t>(tiles_total, 1) * sizeof(double));

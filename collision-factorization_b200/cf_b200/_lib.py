@@ -41,7 +41,8 @@ EXPORTS = [
     "cf_mlp_create", "cf_mlp_destroy", "cf_mlp_num_params", "cf_mlp_copy", "cf_mlp_forward", "cf_mlp_backward",
     "cf_mlp_adam_step", "cf_precond_probe_loss", "cf_precond_assemble",
     "cf_pack_cells", "cf_unpack_cells", "cf_q_tiled", "cf_jv_tiled", "cf_plan_set_kernel_path", "cf_fp64_fma_peak",
-    "cf_status_string", "cf_last_error", "cf_launch_count", "cf_few_route_last", "cf_version",
+    "cf_status_string", "cf_last_error", "cf_launch_count", "cf_few_route_last", "cf_pinned_bytes",
+    "cf_version",
 ]
 
 
@@ -147,6 +148,7 @@ def load(path: str | Path | None = None) -> C.CDLL:
     lib.cf_last_error.restype = C.c_char_p
     lib.cf_launch_count.restype = C.c_int64
     lib.cf_few_route_last.restype = C.c_int
+    lib.cf_pinned_bytes.restype = C.c_int64
     lib.cf_version.restype = C.c_char_p
     lib.cf_plan_last_kernel.restype = C.c_char_p
     lib.cf_plan_last_kernel.argtypes = [C.c_void_p]

@@ -155,6 +155,7 @@ struct cf_plan {
     double* h_stage = nullptr;
     size_t stage_bytes = 0;
     size_t direct_bytes = 0;  // pageable bytes that went without
+    size_t stage_refused = 0;  // smallest size that could not be had (0: none)
     std::mutex mu;
     // q2 <-> q3 folded operator (built on first use of CF_FORM_AF_SYM); fold_status != 0 if the
     // COO list is not symmetric in its last two indices
@@ -261,6 +262,15 @@ int upload(T** dst, const std::vector<T>& src, int64_t& bytes) {
     return CF_OK;
 }
 
+std::atomic<size_t> g_stage_bytes{0};  // pinned staging memory of all plans
+
+void free_stage(cf_plan* p) {
+    if (p->h_stage) cudaFreeHost(p->h_stage);
+    g_stage_bytes -= p->stage_bytes;
+    p->h_stage = nullptr;
+    p->stage_bytes = 0;
+}
+
 void free_plan_memory(cf_plan* p);
 void free_plan_memory(cf_plan* p) {
     if (p->rfd) {
@@ -301,7 +311,7 @@ void free_plan_memory(cf_plan* p) {
     if (p->h_xepoch) cudaFreeHost(p->h_xepoch);
     if (p->h_xsync) cudaFreeHost(p->h_xsync);
     if (p->h_few) cudaFreeHost(p->h_few);
-    if (p->h_stage) cudaFreeHost(p->h_stage);
+    free_stage(p);
     if (p->stream) cudaStreamDestroy(p->stream);
     for (cudaStream_t& hs : p->host_streams)
         if (hs) cudaStreamDestroy(hs);
@@ -1371,7 +1381,10 @@ int ensure_stream_sync(cf_plan* p) {
 //     direct): one per MB, six at most; calls under 2 MB go direct.
 //   memory: pinning costs 0.4 ms per MB once and a staged call saves 0.08 ms per MB or more, so a plan goes direct for
 //     the bytes of kStageAfter such calls first (calls that stop there pay nothing, none pays twice the direct time).
+//     It is freed with the plan; all plans together hold at most kStageTotalBytes, and a size that the system
+//     refused is not asked for again.
 constexpr size_t kStageMaxBytes = (size_t)128 << 20;  // pinned memory of a plan, at most; larger calls go direct
+constexpr size_t kStageTotalBytes = (size_t)256 << 20;
 constexpr size_t kStageAfter = 4;
 constexpr size_t kStagePiece = (size_t)256 << 10;
 constexpr int kStageThreads = 6;
@@ -1404,12 +1417,17 @@ class HostStage {
                 p->direct_bytes += need;
                 return;
             }
-            if (p->h_stage) cudaFreeHost(p->h_stage);
-            p->h_stage = nullptr;
-            p->stage_bytes = 0;
+            if (p->stage_refused != 0 && need >= p->stage_refused) return;
+            if (g_stage_bytes.fetch_add(need) + need - p->stage_bytes > kStageTotalBytes) {
+                g_stage_bytes -= need;
+                return;
+            }
+            free_stage(p);
             if (cudaHostAlloc((void**)&p->h_stage, need, cudaHostAllocDefault) != cudaSuccess) {
                 cudaGetLastError();
                 p->h_stage = nullptr;
+                g_stage_bytes -= need;
+                p->stage_refused = need;
                 return;
             }
             p->stage_bytes = need;
@@ -2261,6 +2279,7 @@ const char* cf_status_string(int status) {
 const char* cf_last_error(void) { return g_last_error.c_str(); }
 int64_t cf_launch_count(void) { return g_launches.load(); }
 int cf_few_route_last(void) { return g_few_route; }
+int64_t cf_pinned_bytes(void) { return (int64_t)g_stage_bytes.load(); }
 // The sources' digest (set by build.py) is part of it: the autotuners' caches hold a choice for one set of kernels.
 #ifndef CF_SOURCE_ID
 #define CF_SOURCE_ID "unknown"

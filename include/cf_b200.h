@@ -120,8 +120,8 @@ int cf_radial_first(double* Q, const double* f, const double* labels, const doub
  * whole batch starts as soon as the first chunk of cells is on the device and hands each chunk back
  * as soon as it is final, with the same result bits as the device entry points.  Other forms cut
  * the batch into chunks that go up, are contracted and come back on three streams.  Pageable arrays go
- * through pinned memory of the plan (at most 128 MB, taken once a plan has seen a few such calls) that
- * several threads copy into and out of.  Up to 8 cells
+ * through pinned memory of the plan (at most 128 MB, and 256 MB for all plans, taken once a plan has seen a few such
+ * calls and freed with it; cf_pinned_bytes) that several threads copy into and out of.  Up to 8 cells
  * (one f per call, as the reference's MEX is called), the fast forms CF_FORM_AF, CF_FORM_AF_SYM and
  * CF_FORM_RF (K <= 8 for RF) are one launch of the few-cell kernel, with f and Q_in passed in the
  * launch's parameter block when they fit (2 B N_Q K <= 3968 doubles); cf_angular_first and
@@ -408,6 +408,8 @@ int64_t cf_launch_count(void);
  * few-cell kernel, 1 f and Q_in in the launch's parameter block (Q_out written to mapped pinned
  * memory), 2 copies through pinned staging and a device buffer. */
 int cf_few_route_last(void);
+/* Pinned host memory that the plans of this process hold for staging pageable arrays. */
+int64_t cf_pinned_bytes(void);
 /* Library version string, with a digest of the kernels' sources: what was measured with one version (the
  * autotuners' caches) is not taken over by another. */
 const char* cf_version(void);

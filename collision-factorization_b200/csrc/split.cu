@@ -922,30 +922,43 @@ struct LbRun {
 
 // phi += the n runs at rec, FP64: lane (cell c, part p) holds phi[k2][y], k3 = p KQ + y; fsg + row
 // offset + (c K + k) 8 is f.
+// K = 8: a lane's two k3 are one 16-byte load (8 of them are 512 contiguous bytes; as two 8-byte loads, twice the
+// wavefronts), and a run with one q3 reads its row once: with both halves read, runs of one, two in three of the plain
+// operator's, made it slower than entries taken one by one.  B200, us, entries one by one / two reads / one read / and in 16
+// bytes: L = 8, 2500 cells plain 1270 / 1423 / 1284 / 1169, folded 699 / 690 / 663 / 612; L = 16, 300 cells plain 2803 / 3502 /
+// 3034 / 2615, folded 1257 / 1290 / 1219 / 1043.  K = 12 keeps both reads (plain L = 16, 300 cells: 4930 one by one, 4885).
 template <int K>
 __device__ __forceinline__ void phi_runs(const unsigned char* rec, int n, const unsigned char* fsg, int c, int part,
                                          double (&phi)[K][K / 4]) {
     constexpr int KQ = K / 4;
+    constexpr bool SKIP = KQ == 2;
     const unsigned char* f2c = fsg + c * K * 8;
     const unsigned char* f3c = f2c + part * KQ * 8;
+    auto row = [&](uint32_t off, double (&f)[KQ]) {
+        if constexpr (KQ == 2) {
+            const double2 x = *reinterpret_cast<const double2*>(f3c + off);
+            f[0] = x.x;
+            f[1] = x.y;
+        } else {
+#pragma unroll
+            for (int y = 0; y < KQ; ++y) f[y] = reinterpret_cast<const double*>(f3c + off)[y];
+        }
+    };
     LbRun<double> r;
     r.read(rec);
-    double h[KQ];
+    double h[KQ], fa[KQ], fb[KQ];
+    row(r.off3a, fa);
+    row(r.off3b, fb);
 #pragma unroll
-    for (int y = 0; y < KQ; ++y)
-        h[y] = fma(r.gb, reinterpret_cast<const double*>(f3c + r.off3b)[y],
-                   r.ga * reinterpret_cast<const double*>(f3c + r.off3a)[y]);
+    for (int y = 0; y < KQ; ++y) h[y] = fma(r.gb, fb[y], r.ga * fa[y]);
 #pragma unroll 1
     for (int i = 1; i <= n; ++i) {
         const double2* f2p = reinterpret_cast<const double2*>(f2c + r.off2);
         if (i < n) rec += LbRun<double>::BYTES;  // the last pass reads the last run again
         r.read(rec);
-        double fa[KQ], fb[KQ];
-#pragma unroll
-        for (int y = 0; y < KQ; ++y) {
-            fa[y] = reinterpret_cast<const double*>(f3c + r.off3a)[y];
-            fb[y] = reinterpret_cast<const double*>(f3c + r.off3b)[y];
-        }
+        const bool two = !SKIP || r.off3b != r.off3a;
+        row(r.off3a, fa);
+        if (two) row(r.off3b, fb);
 #pragma unroll
         for (int x = 0; x < K / 2; ++x) {
             const double2 f2 = f2p[x];
@@ -956,7 +969,7 @@ __device__ __forceinline__ void phi_runs(const unsigned char* rec, int n, const 
             }
         }
 #pragma unroll
-        for (int y = 0; y < KQ; ++y) h[y] = fma(r.gb, fb[y], r.ga * fa[y]);
+        for (int y = 0; y < KQ; ++y) h[y] = fma(r.gb, two ? fb[y] : fa[y], r.ga * fa[y]);
     }
 }
 

@@ -94,7 +94,8 @@ struct cf_plan {
     int n_items = 0;
     double flops_q = 0, flops_jv = 0;
     int64_t dev_bytes = 0;
-    // device operator
+    // device operator: arrays in one allocation (PlanArrays)
+    void* d_arrays = nullptr;
     int* d_q1_begin = nullptr;
     int* d_slice_t = nullptr;
     int* d_slice_e = nullptr;
@@ -104,7 +105,7 @@ struct cf_plan {
     float* d_R32 = nullptr;  // FP32 copy of R for CF_FORM_AF_F32
     double* d_RT = nullptr;  // K = 8: R_t as [k1][8 k2 + k3] for the MMA kernel
     unsigned short* d_RTbf = nullptr;  // K = 8: the same split into BF16 hi and lo parts
-    double2* d_x_R = nullptr;  // outer-product kernels' tables (build_outer), one allocation
+    double2* d_x_R = nullptr;  // outer-product kernels' tables (outer_tables)
     unsigned char* d_x_chunk = nullptr;
     int4* d_x_slice = nullptr;
     int* d_x_q1 = nullptr;
@@ -253,14 +254,40 @@ int validate(const double* labels, const double* vals, const double* ic_map, con
     return CF_OK;
 }
 
-template <typename T>
-int upload(T** dst, const std::vector<T>& src, int64_t& bytes) {
-    const size_t nb = std::max<size_t>(src.size(), 1) * sizeof(T);
-    CF_CUDA(cudaMalloc((void**)dst, nb));
-    if (!src.empty()) CF_CUDA(cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
-    bytes += (int64_t)nb;
-    return CF_OK;
-}
+// A plan's device arrays, made as one allocation: a cudaMalloc above 2 MB takes 0.35 ms, and its cudaFree about as much.
+class PlanArrays {
+   public:
+    // an array filled from src, which has to live until place(), and an array of n elements left as it is
+    template <typename T>
+    void put(T** dst, const std::vector<T>& src) {
+        add((void**)dst, src.data(), src.size() * sizeof(T));
+    }
+    template <typename T>
+    void room(T** dst, size_t n) {
+        add((void**)dst, nullptr, n * sizeof(T));
+    }
+    int place(cf_plan* p) {
+        CF_CUDA(cudaMalloc(&p->d_arrays, total_));
+        p->dev_bytes = (int64_t)total_;
+        for (const Piece& x : pieces_) *x.dst = (char*)p->d_arrays + x.at;
+        for (const Piece& x : pieces_)
+            if (x.src && x.bytes) CF_CUDA(cudaMemcpy(*x.dst, x.src, x.bytes, cudaMemcpyHostToDevice));
+        return CF_OK;
+    }
+
+   private:
+    struct Piece {
+        void** dst;
+        const void* src;
+        size_t bytes, at;
+    };
+    void add(void** dst, const void* src, size_t bytes) {
+        pieces_.push_back({dst, src, bytes, total_});
+        total_ += (std::max<size_t>(bytes, 1) + 255) & ~(size_t)255;
+    }
+    std::vector<Piece> pieces_;
+    size_t total_ = 0;
+};
 
 std::atomic<size_t> g_stage_bytes{0};  // pinned staging memory of all plans
 
@@ -286,25 +313,7 @@ void free_plan_memory(cf_plan* p) {
         delete p->sym;
         p->sym = nullptr;
     }
-    cudaFree(p->d_q1_begin);
-    cudaFree(p->d_slice_t);
-    cudaFree(p->d_slice_e);
-    cudaFree(p->d_e_q23);
-    cudaFree(p->d_e_g);
-    cudaFree(p->d_R);
-    cudaFree(p->d_R32);
-    cudaFree(p->d_RT);
-    cudaFree(p->d_RTbf);
-    cudaFree(p->d_x_R);
-    cudaFree(p->d_item_cum);
-    cudaFree(p->d_item_q1);
-    cudaFree(p->d_bin_begin);
-    cudaFree(p->d_bin_q1);
-    cudaFree(p->d_counter);
-    cudaFree(p->d_pbin_begin);
-    cudaFree(p->d_pbin_item);
-    cudaFree(p->d_pair_cum);
-    cudaFree(p->d_pitems);
+    cudaFree(p->d_arrays);
     cudaFree(p->d_ws);
     cudaFree(p->d_io);
     cudaFree(p->d_xready);
@@ -323,15 +332,22 @@ void free_plan_memory(cf_plan* p) {
 
 // Tables of the outer-product kernels (outer_kernels.cuh).  The host counts every slice's runs (equal q2, one or two
 // entries) and places its chunks of four; the chunks themselves are packed on the device (pack_chunks_kernel), as
-// every plan has them made, also one whose fast forms are never called: a plan's making takes 3.5 ms at L = 10, K = 8
-// (packed on one host thread 5.0; without these tables, and all copies of R made on the host, 3.8).
-int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<int>& slice_t,
-                const std::vector<int>& slice_e, const std::vector<uint32_t>& e_q23, int64_t& bytes) {
-    const size_t S = slice_t.size();
-    std::vector<int4> xs, place(S);  // place: first chunk, runs of two, runs
-    std::vector<int> xbegin(S + 1, 0), xq1(q1_begin.size()), count(p->n_q, 0);
-    xs.reserve(S + S / 8);
+// every plan has them made, also one whose fast forms are never called: with all arrays in one allocation a plan's making
+// takes 2.5 ms at L = 10, K = 8 and 1.3 ms at L = 8, K = 7 (without these tables and with an allocation per array 4.1 and
+// 1.15; with them, packed on one host thread, 5.2 and 2.1).
+struct OuterTables {
+    std::vector<int4> slices, place;  // place: first chunk, runs of two, runs
+    std::vector<int> q1;
     int n_chunks = 0;
+};
+OuterTables outer_tables(int n_q, const std::vector<int>& q1_begin, const std::vector<int>& slice_t,
+                         const std::vector<int>& slice_e, const std::vector<uint32_t>& e_q23) {
+    OuterTables x;
+    const size_t S = slice_t.size();
+    std::vector<int> xbegin(S + 1, 0), count(n_q, 0);
+    x.place.resize(S);
+    x.q1.resize(q1_begin.size());
+    x.slices.reserve(S + S / 8);
     for (size_t s = 0; s < S; ++s) {
         for (int e = slice_e[s]; e < slice_e[s + 1]; ++e) ++count[e_q23[e] & 0xffffu];
         int n_two = 0, n_all = 0;
@@ -341,43 +357,17 @@ int build_outer(cf_plan* p, const std::vector<int>& q1_begin, const std::vector<
             n_all += (c + 1) / 2;
             c = 0;
         }
-        place[s] = make_int4(n_chunks, n_two, n_all, 0);
+        x.place[s] = make_int4(x.n_chunks, n_two, n_all, 0);
         // a ring stage holds kOuterChunks chunks; the K^3 step is linear, so a longer slice is several
         const int n = (n_all + 3) / 4, n2 = (n_two + 3) / 4;
         for (int c = 0; c < n; c += cf::kOuterChunks)
-            xs.push_back(make_int4(slice_t[s], n_chunks + c, std::max(0, std::min(cf::kOuterChunks, n2 - c)),
-                                   std::min(cf::kOuterChunks, n - c)));
-        n_chunks += n;
-        xbegin[s + 1] = (int)xs.size();
+            x.slices.push_back(make_int4(slice_t[s], x.n_chunks + c, std::max(0, std::min(cf::kOuterChunks, n2 - c)),
+                                         std::min(cf::kOuterChunks, n - c)));
+        x.n_chunks += n;
+        xbegin[s + 1] = (int)x.slices.size();
     }
-    for (size_t q = 0; q < q1_begin.size(); ++q) xq1[q] = xbegin[q1_begin[q]];
-    // one allocation: R_t in lane order, the chunks, then what the host made
-    const size_t nR = (size_t)p->n_l * p->k * 32, b_R = nR * sizeof(double2), b_ch = (size_t)n_chunks * cf::kOuterChunkWords * 8;
-    const size_t b_xs = xs.size() * sizeof(int4), b_pl = S * sizeof(int4), b_q1 = xq1.size() * sizeof(int);
-    std::vector<unsigned char> host(b_xs + b_pl + b_q1);
-    if (b_xs) std::memcpy(host.data(), xs.data(), b_xs);
-    if (b_pl) std::memcpy(host.data() + b_xs, place.data(), b_pl);
-    std::memcpy(host.data() + b_xs + b_pl, xq1.data(), b_q1);
-    unsigned char* d = nullptr;
-    CF_CUDA(cudaMalloc((void**)&d, b_R + b_ch + host.size()));
-    p->d_x_R = (double2*)d;
-    p->d_x_chunk = d + b_R;
-    p->d_x_slice = (int4*)(d + b_R + b_ch);
-    const int4* d_place = p->d_x_slice + xs.size();
-    p->d_x_q1 = (int*)(d_place + S);
-    bytes += (int64_t)(b_R + b_ch + host.size());
-    CF_CUDA(cudaMemcpy(d + b_R + b_ch, host.data(), host.size(), cudaMemcpyHostToDevice));
-    const int n_zero = cf::outer_zeros(p->n_q, cf::outer_nqp(cf::outer_fit(p->n_q, p->k, false, p->max_smem).width));
-    if (S > 0) {
-        cf::pack_chunks_kernel<<<(unsigned)((S + 63) / 64), 64>>>(p->d_slice_e, p->d_e_q23, p->d_e_g, d_place, (int)S, p->n_q,
-                                                                 n_zero, (unsigned long long*)p->d_x_chunk);
-        CF_CUDA(cudaGetLastError());
-    }
-    if (nR > 0) {
-        cf::lane_order_kernel<<<(unsigned)((nR + 255) / 256), 256>>>(p->d_R, p->d_x_R, nR, p->k);
-        CF_CUDA(cudaGetLastError());
-    }
-    return CF_OK;
+    for (size_t q = 0; q < q1_begin.size(); ++q) x.q1[q] = xbegin[q1_begin[q]];
+    return x;
 }
 
 // Build the q1-grouped run structure (host) and upload it.
@@ -500,57 +490,69 @@ int build_plan(cf_plan* p, const double* labels, const double* vals, const doubl
 
     std::vector<double> Rv((size_t)K * K * K * p->n_l);
     if (NG > 0) std::memcpy(Rv.data(), R, Rv.size() * sizeof(double));
-    int64_t bytes = 0;
-    CF_TRY(upload(&p->d_q1_begin, q1_begin, bytes));
-    CF_TRY(upload(&p->d_slice_t, slice_t, bytes));
-    CF_TRY(upload(&p->d_slice_e, slice_e, bytes));
-    CF_TRY(upload(&p->d_e_q23, e_q23, bytes));
-    CF_TRY(upload(&p->d_e_g, e_g, bytes));
-    CF_TRY(upload(&p->d_R, Rv, bytes));
-    {
-        // the other copies of R are made from it on the device
-        const size_t n = Rv.size(), n8 = K == 8 ? n : 0;
-        CF_CUDA(cudaMalloc((void**)&p->d_R32, std::max<size_t>(n, 1) * sizeof(float)));
-        if (n8) {
-            CF_CUDA(cudaMalloc((void**)&p->d_RT, n * sizeof(double)));
-            CF_CUDA(cudaMalloc((void**)&p->d_RTbf, 2 * n * sizeof(unsigned short)));
-        }
-        bytes += (int64_t)(n * sizeof(float) + n8 * (sizeof(double) + 2 * sizeof(unsigned short)));
-        if (n) {
-            cf::derive_r_kernel<<<(unsigned)((n + 255) / 256), 256>>>(p->d_R, p->d_R32, p->d_RT, p->d_RTbf, n);
-            CF_CUDA(cudaGetLastError());
-        }
-    }
-    CF_TRY(upload(&p->d_item_q1, items, bytes));
     // the rows' work in list order, added up: an entry K^2 FMAs, a slice K^3, a row's end about as much
-    std::vector<long long> item_cum(1, 0);
-    for (int q : items)
-        item_cum.push_back(item_cum.back() + (long long)(q1_begin[q + 1] - q1_begin[q] + 1) * K +
-                           slice_e[q1_begin[q + 1]] - slice_e[q1_begin[q]]);
-    CF_TRY(upload(&p->d_item_cum, item_cum, bytes));
-    CF_TRY(upload(&p->d_bin_begin, bin_begin, bytes));
-    CF_TRY(upload(&p->d_bin_q1, bin_q1, bytes));
-    CF_TRY(upload(&p->d_pbin_begin, pbin_begin, bytes));
-    CF_TRY(upload(&p->d_pbin_item, pbin_item, bytes));
-    std::vector<long long> pair_cum(1, 0);
-    for (int i : porder) {
-        const int q = pitems[i].x;
-        pair_cum.push_back(pair_cum.back() + (long long)(q1_begin[q + 1] - q1_begin[q] + 1) * K +
-                           slice_e[q1_begin[q + 1]] - slice_e[q1_begin[q]]);
-    }
-    CF_TRY(upload(&p->d_pair_cum, pair_cum, bytes));
-    CF_TRY(upload(&p->d_pitems, pitems, bytes));
-    CF_CUDA(cudaMalloc((void**)&p->d_counter, kCounterSlots * sizeof(int)));
-    bytes += kCounterSlots * sizeof(int);
+    auto row_work = [&](int q) {
+        return (long long)(q1_begin[q + 1] - q1_begin[q] + 1) * K + slice_e[q1_begin[q + 1]] - slice_e[q1_begin[q]];
+    };
+    std::vector<long long> item_cum(1, 0), pair_cum(1, 0);
+    for (int q : items) item_cum.push_back(item_cum.back() + row_work(q));
+    for (int i : porder) pair_cum.push_back(pair_cum.back() + row_work(pitems[i].x));
     int dev = 0, optin = 0;
     CF_CUDA(cudaGetDevice(&dev));
     CF_CUDA(cudaDeviceGetAttribute(&p->n_sms, cudaDevAttrMultiProcessorCount, dev));
     CF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     p->max_smem = (size_t)optin;
-    if (cf::outer_for(K) && cf::outer_fit(NQ, K, false, p->max_smem).nc > 0)
-        CF_TRY(build_outer(p, q1_begin, slice_t, slice_e, e_q23, bytes));
+    const cf::OuterFit fit = cf::outer_for(K) ? cf::outer_fit(NQ, K, false, p->max_smem) : cf::OuterFit{0, 0};
+    OuterTables outer;
+    if (fit.nc > 0) outer = outer_tables(NQ, q1_begin, slice_t, slice_e, e_q23);
+
+    PlanArrays arrays;
+    arrays.put(&p->d_q1_begin, q1_begin);
+    arrays.put(&p->d_slice_t, slice_t);
+    arrays.put(&p->d_slice_e, slice_e);
+    arrays.put(&p->d_e_q23, e_q23);
+    arrays.put(&p->d_e_g, e_g);
+    arrays.put(&p->d_R, Rv);
+    arrays.put(&p->d_item_q1, items);
+    arrays.put(&p->d_item_cum, item_cum);
+    arrays.put(&p->d_bin_begin, bin_begin);
+    arrays.put(&p->d_bin_q1, bin_q1);
+    arrays.put(&p->d_pbin_begin, pbin_begin);
+    arrays.put(&p->d_pbin_item, pbin_item);
+    arrays.put(&p->d_pair_cum, pair_cum);
+    arrays.put(&p->d_pitems, pitems);
+    arrays.room(&p->d_counter, kCounterSlots);
+    // the other copies of R, and the chunks, are made on the device
+    const size_t n = Rv.size(), nR = (size_t)p->n_l * K * 32, S_x = outer.place.size();
+    arrays.room(&p->d_R32, n);
+    if (K == 8) {
+        arrays.room(&p->d_RT, n);
+        arrays.room(&p->d_RTbf, 2 * n);
+    }
+    int4* d_place = nullptr;
+    if (fit.nc > 0) {
+        arrays.put(&p->d_x_slice, outer.slices);
+        arrays.put(&p->d_x_q1, outer.q1);
+        arrays.put(&d_place, outer.place);
+        arrays.room(&p->d_x_R, nR);
+        arrays.room(&p->d_x_chunk, (size_t)outer.n_chunks * cf::kOuterChunkWords * 8);
+    }
+    CF_TRY(arrays.place(p));
+    if (n) {
+        cf::derive_r_kernel<<<(unsigned)((n + 255) / 256), 256>>>(p->d_R, p->d_R32, p->d_RT, p->d_RTbf, n);
+        CF_CUDA(cudaGetLastError());
+    }
+    if (S_x > 0) {
+        cf::pack_chunks_kernel<<<(unsigned)((S_x + 63) / 64), 64>>>(p->d_slice_e, p->d_e_q23, p->d_e_g, d_place, (int)S_x, NQ,
+                                                                   cf::outer_zeros(NQ, cf::outer_nqp(fit.width)),
+                                                                   (unsigned long long*)p->d_x_chunk);
+        CF_CUDA(cudaGetLastError());
+    }
+    if (fit.nc > 0 && nR > 0) {
+        cf::lane_order_kernel<<<(unsigned)((nR + 255) / 256), 256>>>(p->d_R, p->d_x_R, nR, K);
+        CF_CUDA(cudaGetLastError());
+    }
     CF_CUDA(cudaStreamSynchronize(nullptr));  // a launch on another stream may read what the kernels here wrote
-    p->dev_bytes = bytes;
     return CF_OK;
 }
 

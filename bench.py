@@ -727,7 +727,7 @@ def run_e2e(op, geo, R, cells, K, args, world, form="af"):
             "form": form,
             "path": "cf_contract_host (the MEX-compatible host entry point: content-keyed plan cache, checked while "
                     "the GPU works from the second call on; the folded fast form at K <= 8 streams the batch through one "
-                    "tile-kernel launch while chunks are copied in and out, other forms run the chunked pipeline on "
+                    "launch while chunks are copied in and out, other forms run the chunked pipeline on "
                     "three streams), pinned host buffers, Q_out zeroed by one host thread before each call (outside "
                     "the timing)"}
 

@@ -19,7 +19,7 @@
 // grid-wide step between them, and the basis is read three times (h; w' = w - V h with V^T w' in the same
 // pass; w'' = w' - V hh) instead of four.  Cells converge at different steps; once a quarter of them are
 // done, J.v runs on the active cells gathered into whole tiles.
-// B200, L = 8, K = 8, 2048 cells, dt nu = 10, block preconditioner: 8.6 ms a solve, 6.9 of them J.v and 1.0 k_step;
+// B200, L = 8, K = 8, 2048 cells, dt nu = 10, block preconditioner: 8.0 ms a solve, 6.4 of them J.v and 1.0 k_step;
 // 16.8 ms with one launch per vector operation on 64 CTAs (k_dots alone 5.6 ms) and J.v of every cell until the
 // last had converged (8 to 14 steps).
 #include <cuda_runtime.h>

@@ -115,10 +115,12 @@ int cf_radial_first(double* Q, const double* f, const double* labels, const doub
 
 /* Batched host-pointer form of both (Q, f: [N_Q x K x B]); form is a cf_form.  The host-side
  * counterpart of calling the reference MEX once per cell (benchmark_collision_contraction_scaling.m:96-108).
- * From 512 cells up, the fast FP64 forms that run on the tile kernel (CF_FORM_AF_SYM with the
- * automatic kernel order; either fast form with kernel path 2) are streamed: one launch over the
- * whole batch starts as soon as the first chunk of cells is on the device and hands each chunk back
- * as soon as it is final, with the same result bits as the device entry points.  Other forms cut
+ * From 512 cells up, the fast FP64 forms at even K <= 8 that run on the tile kernel or, at K = 8, on 16-cell units
+ * of the outer-product kernel (CF_FORM_AF_SYM with the automatic kernel order; either fast form with kernel path 2)
+ * are streamed: one launch over the
+ * whole batch, queued behind all its uploads, starts as soon as the first chunk of cells is on the device
+ * (pageable arrays: once the last chunk has been copied into pinned memory or to the device) and hands each
+ * chunk back as soon as it is final, with the same result bits as the device entry points.  Other forms cut
  * the batch into chunks that go up, are contracted and come back on three streams.  Pageable arrays go
  * through pinned memory of the plan (at most 128 MB, and 256 MB for all plans, taken once a plan has seen a few such
  * calls and freed with it; cf_pinned_bytes) that several threads copy into and out of.  Up to 8 cells

@@ -500,7 +500,7 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
     if (a.ss) {
         if (a.what == OP_RF || a.exact || a.f32) return {8, 0, cudaSuccess, PATH_TILE};
         if constexpr (outer_for(K)) {
-            if (a.path == PATH_AUTO && outer_takes(K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms)) {
+            if (a.path == PATH_AUTO && outer_takes(a.op.n_q, K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms, a.max_smem)) {
                 const LaunchResult r = a.what == OP_JV ? launch_outer<K, true>(a) : launch_outer<K, false>(a);
                 if (r.status != -1) return r;
             }
@@ -564,7 +564,7 @@ static LaunchResult launch_for_k(const LaunchArgs& a) {
         return launch_for_k<K>(b);
     }
     if constexpr (outer_for(K)) {
-        if (a.path == PATH_AUTO && !a.exact && outer_takes(K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms)) {
+        if (a.path == PATH_AUTO && !a.exact && outer_takes(a.op.n_q, K, a.tile_first, a.what == OP_JV, a.n_cells, a.n_sms, a.max_smem)) {
             const LaunchResult r = jv ? launch_outer<K, true>(a) : launch_outer<K, false>(a);
             if (r.status != -1) return r;
         }

@@ -117,12 +117,17 @@ constexpr int kTileBufs = 4;  // half-tiles that a CTA of the tile kernel holds 
 // K that the outer-product kernels (outer_kernels.cuh) take.
 constexpr bool outer_for(int K) { return K >= 7 && K <= 8; }
 
-// Where they are the faster family (B200, us, outer / tile or pair): nearly everywhere (folded Q, K = 8: L = 10, 4096
-// cells 1509 / 1642, L = 13, 1000 cells 1045 / 1928, L = 6, 2048 cells 161 / 176, L = 3, 2000 cells 39 / 51; J.v, L = 10,
-// 2174 / 3060; plain Q, K = 7, L = 5, 4096 cells 250 / 266).  The pair kernel keeps the plain J.v at K = 7 on batches of more
-// than two thirds of a half-tile per SM (L = 8: 4096 cells 1677 / 1570, 1300 cells 571 / 691; L = 6, 2000 cells: 312 / 299).
-constexpr bool outer_takes(int K, bool folded, bool jv, int64_t n_cells, int n_sms) {
-    return outer_for(K) && (K == 8 || folded || !jv || (n_cells + 15) / 16 * 3 <= 2 * n_sms);
+// Where they are taken: every fast form at these K but the plain J.v at K = 7 on batches of more than two thirds of a half-tile
+// per SM, which stays on the pair kernel where that fits (it does not at L = 10: 2000 cells 1944 us, 3084 on the gather kernel
+// otherwise).  But for that one form the kernel, and so a cell's bits, does not depend on the batch.
+// The faster family (B200, us, outer / the better of tile and pair): on small batches at every size (20 cells, L = 3 17.4 /
+// 17.4, L = 6 22.5 / 28.7, L = 10 39.9 / 57.5, K = 8 folded Q), on large ones from L = 8 on at K = 8 (4096 cells, folded Q: L = 8
+// 705 / 711, L = 10 1520 / 1624; J.v L = 8 980 / 1009; plain Q L = 8 1254 / 1254, L = 10 2832 / 3011; L = 13, 1000 cells 1055 /
+// 1928) and for the folded Q at K = 7 (646 / 668).  Below, the tile and pair kernels in stretches are the faster ones (4096
+// cells, K = 8 folded Q: L = 6 290 / 261, L = 3 63 / 45; K = 7 plain Q: L = 5 253 / 191, L = 8 1150 / 982), but only
+// from a hundred to six hundred cells on.
+constexpr bool outer_takes(int n_q, int K, bool folded, bool jv, int64_t n_cells, int n_sms, size_t max_smem) {
+    return outer_for(K) && (K == 8 || folded || !jv || (n_cells + 15) / 16 * 3 <= 2 * n_sms || pair_fit(n_q, K, true, max_smem) == 0);
 }
 
 // Shared-memory geometry of the outer-product kernels.  Cells lie in pairs, [pair][k][q][cell of the pair],

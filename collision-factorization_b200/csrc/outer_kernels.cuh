@@ -22,8 +22,8 @@
 // What bounds it: shared-memory wavefronts (72 % of peak at L = 10, K = 8: 17 a cell and slice for the Phi operands,
 // 8 for R_t, 8 for chunks, heads and copies), with the FP64 pipe at 50 %.  Four cells a warp (128 registers,
 // 16 warps) rather than eight (255, 8 warps, half the R_t wavefronts): 1591 against 1847 us, latency; R_t read
-// from L2 by each warp instead of staged: 2184 us.  B200, folded, L = 10, K = 8, 4096 cells: Q 1509 us (tile kernel
-// 1642), J.v 2174 us (quarter-tile kernel 3060); L = 13, 1000 cells: Q 1045 us (1928); L = 10, 300 cells: 158 us (285).
+// from L2 by each warp instead of staged: 2184 us.  B200, folded, L = 10, K = 8, 4096 cells: Q 1520 us (tile kernel
+// 1624), J.v 2185 us (quarter-tile kernel 3060); L = 13, 1000 cells: Q 1057 us (1928); L = 10, 300 cells: 157 us (232).
 #pragma once
 #include <type_traits>
 

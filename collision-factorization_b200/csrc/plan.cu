@@ -763,7 +763,7 @@ int run_device(cf_plan* p, int what, bool exact, double* q_dev, const double* f_
     if (ws_bytes < need) return fail(CF_EINVAL, "workspace of %zu bytes is smaller than %zu", ws_bytes, need);
     // The fast FP64 Q and J.v forms on the outer-product kernel: one launch on the cell-major arrays.
     if (!exact && f32 == 0 && (what == 0 || what == 2) && p->path == cf::PATH_AUTO &&
-        cf::outer_takes(p->k, sym, what == 2, B, p->n_sms) &&
+        cf::outer_takes(p->n_q, p->k, sym, what == 2, B, p->n_sms, p->max_smem) &&
         cf::outer_fit(p->n_q, p->k, what == 2, p->max_smem).nc > 0) {
         cf_plan* target = p;
         if (sym) CF_TRY(get_sym(p, &target));

@@ -268,8 +268,8 @@ int cf_plan_lblock_selftest(cf_plan* plan, double wait_seconds);
  * pair routine (8 warps per CTA), 1 the tile routine (16 warps per CTA; buckets of odd K then run
  * on their own).  tail_split (0, 4 or 16) is how many bins each of the last half-tiles of the fused
  * work table is cut into, so that the launch ends evenly (0: none is cut); the one launch on the
- * cell-major arrays cuts the half-tiles that would outlast a CTA's share of the step's work, into
- * that many bins or 16.
+ * cell-major arrays takes the table that is the shorter by estimate of two: that one, or one that cuts the
+ * half-tiles which would outlast a CTA's share of the step's work, into that many bins or 16.
  * cf_ragged_q enqueues pack, fused launch, the separate buckets and unpack on the stream (when every
  * non-empty bucket is fused on the tile routine: one launch on the cell-major arrays instead);
  * cf_ragged_graph_launch records that sequence into a CUDA graph on first use (per set of buffers)
